@@ -53,18 +53,21 @@ __device__ __forceinline__ int32_t sat_bin(float r) {
     return (int32_t)__float2uint_rz(r);
 }
 
-// rint(fl(mz / 1.0005079)).  A multiply by the rounded reciprocal lies within
-// 2^-22 relative of the IEEE quotient, i.e. within 2^-8 for |q| < 2^14; when
-// it is farther than 1/128 from a half-integer -- its distance to the nearest
-// integer, |q - rint(q)| (exact), is below 1/2 - 1/128 -- both round to the
-// same integer, otherwise the IEEE quotient itself is computed.  Exact.
+// rint(fl(mz / 1.0005079)).  q, the product with the rounded reciprocal, lies
+// within |q| 2^-22 of the IEEE quotient (three roundings of 2^-24 relative
+// each); when q is farther than |q| 2^-21 from every half-integer -- its
+// distance to the nearest integer, |q - rint(q)| (exact), is below
+// 1/2 - |q| 2^-21 -- both round to the same integer, otherwise the IEEE
+// quotient itself is computed.  Exact.  (A fixed distance of 1/128, good for
+// every |q| < 2^14, sent one lane in 64 to the division and with it most
+// warps; at a bin of 1,000 this sends one in 1,000.)
 constexpr float kInvBinMono = 1.0f / 1.0005079f;
 template <bool FastDiv>
 __device__ __forceinline__ int32_t bin_of(float mz) {
     if constexpr (FastDiv) return sat_bin(rintf(__fdividef(mz, kBinMono)));
     const float q = __fmul_rn(mz, kInvBinMono);
     const float r = rintf(q);
-    if (fabsf(q) < 16384.0f && fabsf(__fsub_rn(q, r)) < 0.4921875f) return sat_bin(r);
+    if (fabsf(__fsub_rn(q, r)) < __fmaf_rn(fabsf(q), -0x1p-21f, 0.5f)) return sat_bin(r);
     return sat_bin(rintf(__fdiv_rn(mz, kBinMono)));
 }
 

@@ -566,16 +566,16 @@ int32_t search_isoform_lists(hfx_ctx *ctx, const hfx_search_params *p, const Spe
     uint16_t *lists = e ? nullptr : ctx->buf<uint16_t>("i_lists", cap_entries + 64, e);
     const int32_t pos_words = (int32_t)((ctx->max_ladder + 31) / 32 + 1);
     uint32_t *pos = e ? nullptr : ctx->buf<uint32_t>("i_pos", (cap_iso + 1) * (size_t)pos_words, e);
+    uint32_t *work = e ? nullptr : ctx->buf<uint32_t>("i_work", hfx_lists_work_words(cap_iso), e);
     if (e) return cuda_fail(ctx, e, "alloc isoform lists");
     rc = hfx_iso_expand(db, dm, cover, ctx->d_lstart.as<uint32_t>(), count, incl, units, iunits, (uint32_t)cap_iso,
                         cap_entries, key, off, ctx->d_err.as<uint32_t>(), ctx->stream);
     if (!rc)
         rc = hfx_iso_generate(db, dm, cover, (int32_t)std::min<int64_t>(stride, kMaxWords * 32),
                               ctx->d_lstart.as<uint32_t>(), incl + n, (uint32_t)cap_iso, key, off, lists, cap_entries,
-                              len, (int32_t)std::min<uint64_t>(40ull * ctx->max_ladder, kMaxListLen), pos_words,
-                              pos, p->fastdiv, stats, ctx->d_err.as<uint32_t>(), ctx->stream);
+                              len, pos_words, pos, work, p->fastdiv, stats, ctx->d_err.as<uint32_t>(), ctx->stream);
     if (rc) return cuda_fail(ctx, (cudaError_t)rc, "isoform lists");
-    ctx->stage_end(HFX_STAGE_MOD_LISTS, 17, (int64_t)cap_iso);  // windows, planning, 12 isoform-list kernels
+    ctx->stage_end(HFX_STAGE_MOD_LISTS, 19, (int64_t)cap_iso);  // windows, planning, 14 isoform-list kernels
     ctx->stage_begin(HFX_STAGE_MODS);
     rc = hfx_iso_score(lists, cap_entries, ctx->d_lstart.as<uint32_t>(), key, off, len, count, incl,
                        (uint32_t)ctx->num_pep, (uint32_t)cap_iso, elem_kind, tiles, stride, mb, me, ctx->num_mod, ws,
@@ -688,7 +688,6 @@ int32_t search_batched(hfx_ctx *ctx, const hfx_search_params *p, const Batch &b,
     const void *lists_out = nullptr;  // the step's lists, which the FP32 rescoring reads
     const uint16_t *llen_out = nullptr;
     uint64_t total10_out = 0;
-    const int32_t list_cap = (int32_t)std::min<uint64_t>(40ull * ctx->max_ladder, kMaxListLen);
     const bool mods_on = p->search_mods != 0 && ctx->num_mod > 0;
     ctx->stage_begin(HFX_STAGE_PACK);
     rc = hfx_pack_tiles(src_rows, elem_kind, stride, meta, ws, tiles, ngroups, G, ctx->stream);
@@ -712,6 +711,8 @@ int32_t search_batched(hfx_ctx *ctx, const hfx_search_params *p, const Batch &b,
         int32_t *partial = ctx->buf<int32_t>("l_partial", hfx_scan_partials_needed(kLevels * npep1), e);
         if (e) return cuda_fail(ctx, e, "alloc");
         uint16_t *llen = ctx->buf<uint16_t>("l_len", (size_t)kLevels * ctx->num_pep, e);
+        if (e) return cuda_fail(ctx, e, "alloc");
+        uint32_t *work = ctx->buf<uint32_t>("l_work", hfx_lists_work_words(ctx->num_pep), e);
         if (e) return cuda_fail(ctx, e, "alloc");
         // static slots: 10 ions per prefix and charge (rounded up to 8
         // entries per fragment), levels 1..4 (1+2+3+4)
@@ -738,10 +739,10 @@ int32_t search_batched(hfx_ctx *ctx, const hfx_search_params *p, const Batch &b,
                                          ctx->d_err.as<uint32_t>(), ctx->stream);
         else if (!rc)
             rc = hfx_lists_generate(db, cover, npep1, (int32_t)std::min<int64_t>(stride, kMaxWords * 32),
-                                    ctx->d_lstart.as<uint32_t>(), total10, (uint16_t *)lists, llen, list_cap,
-                                    p->fastdiv, stats, ctx->d_err.as<uint32_t>(), ctx->stream);
+                                    ctx->d_lstart.as<uint32_t>(), total10, (uint16_t *)lists, llen, work,
+                                    p->fastdiv, stats, ctx->stream);
         if (rc) return cuda_fail(ctx, (cudaError_t)rc, "ion lists");
-        ctx->stage_end(HFX_STAGE_LISTS, 5, 0);
+        ctx->stage_end(HFX_STAGE_LISTS, long_rows ? 5 : 8, 0);
         ctx->stage_begin(HFX_STAGE_SCORE);
         float *sink = nullptr;
         const uint64_t *sink_off = nullptr;

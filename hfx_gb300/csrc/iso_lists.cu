@@ -36,6 +36,7 @@
 #include "batched_common.cuh"
 #include "lists.h"
 #include "lists_device.cuh"
+#include "scan.cuh"
 #include "mods_device.cuh"
 #include "iso_lists.h"
 
@@ -161,24 +162,20 @@ __global__ void k_iso_expand(DevDB db, const int32_t *__restrict__ count, const 
 // ModIsoform::chunk_add's, residue by residue; consecutive records are
 // mostly the ranks of one (combination, peptide), so a warp's threads run
 // the same loops.
-__global__ void __launch_bounds__(256) k_iso_positions(DevDB db, DevMods mods, const int32_t *__restrict__ total_p,
-                                                       uint32_t cap_iso, const uint64_t *__restrict__ iso_key,
-                                                       int32_t pos_words, uint32_t *__restrict__ iso_pos,
-                                                       uint32_t *__restrict__ err) {
-    const uint32_t total = min((uint32_t)*total_p, cap_iso);
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= total) return;
-    const uint64_t key = iso_key[t];
+// Returns the record's list class (lists_device.cuh), -1 for a skipped record.
+__device__ __forceinline__ int iso_positions(const DevDB &db, const DevMods &mods, uint64_t key, uint32_t t,
+                                             int32_t pos_words, uint32_t *__restrict__ iso_pos,
+                                             uint32_t *__restrict__ err) {
     const int32_t mu = (int32_t)((key >> 54) & 0x1FFu);
     const uint32_t p = (uint32_t)((key >> 27) & 0x7FFFFFFu), rank = (uint32_t)(key & 0x7FFFFFFu);
     uint32_t *bits = iso_pos + (size_t)t * pos_words;
-    if (key == ~0ull || p >= db.num_pep || mu >= mods.num_mod) return;  // a skipped record
+    if (key == ~0ull || p >= db.num_pep || mu >= mods.num_mod) return -1;  // a skipped record
     const uint32_t tc = db.tc_sorted[p], tn = db.tn_sorted[p];
     const int num_ma = mods.num_ma;
     if (tn > tc && (int64_t)(tn - tc) > 32ll * pos_words) {  // longer than the database's longest peptide
         atomicOr(err, kErrBounds);
         for (int i = 0; i < pos_words; ++i) bits[i] = 0u;
-        return;
+        return -1;
     }
     // modable-acid counts (filter_by_mod.cu:216-230)
     uint32_t D[kMaxMa];
@@ -196,7 +193,7 @@ __global__ void __launch_bounds__(256) k_iso_positions(DevDB db, DevMods mods, c
     if (rank >= niso || !isoform_masks(D, scan, dcount, num_ma, rank, mask)) {
         atomicOr(err, kErrKeyOverflow);
         for (int i = 0; i < pos_words; ++i) bits[i] = 0u;
-        return;
+        return list_class(tc, tn);
     }
     // the i-th acid counter, in peptide order
     uint32_t seen_any = 0u, seen[kMaxMa];
@@ -225,46 +222,59 @@ __global__ void __launch_bounds__(256) k_iso_positions(DevDB db, DevMods mods, c
             word = 0u;
         }
     }
+    return list_class(tc, tn);
 }
 
-// 4b. one warp per isoform: the distinct-bin list of every needed level.
-template <bool FastDiv>
-__global__ void __launch_bounds__(256) k_gen_iso_lists(DevDB db, DevMods mods, const int32_t *__restrict__ cover,
+__global__ void __launch_bounds__(256) k_iso_positions(DevDB db, DevMods mods, const int32_t *__restrict__ total_p,
+                                                       uint32_t cap_iso, const uint64_t *__restrict__ iso_key,
+                                                       int32_t pos_words, uint32_t *__restrict__ iso_pos,
+                                                       WorkLists wl, uint16_t *__restrict__ iso_len,
+                                                       uint32_t *__restrict__ err) {
+    const uint32_t total = min((uint32_t)*total_p, cap_iso);
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    int cls = -1;
+    if (t < total) {
+        cls = iso_positions(db, mods, iso_key[t], t, pos_words, iso_pos, err);
+        if (cls < 0)
+            for (int z = 0; z < kLevels; ++z) iso_len[(size_t)t * kLevels + z] = 0;
+    }
+    append_work(wl, cls, t);
+}
+
+// 4b. one warp per isoform: the distinct-bin list of every needed level
+// (build_lists; classes as in k_gen_lists).  The 3.93 M lists (1.17 G
+// entries) of 1,000 spectra against 5,000 proteins: 5.57 ms by bit planes,
+// 4.15 ms by rank.
+template <bool FastDiv, int NC>
+__global__ void __launch_bounds__(256, NC == 0 ? 1 : 4) k_gen_iso_lists(DevDB db, DevMods mods, const int32_t *__restrict__ cover,
                                                        int64_t npep1, int32_t nbins,
                                                        const uint32_t *__restrict__ lstart,
-                                                       const int32_t *__restrict__ total_p, uint32_t cap_iso,
                                                        const uint64_t *__restrict__ iso_key,
                                                        const uint64_t *__restrict__ iso_off, uint16_t *__restrict__ lists,
                                                        uint64_t list_total, uint16_t *__restrict__ iso_len,
-                                                       int32_t list_cap, int32_t pos_words,
+                                                       int32_t pos_words,
                                                        const uint32_t *__restrict__ iso_pos,
-                                                       unsigned long long *__restrict__ stats,
+                                                       WorkLists wl, unsigned long long *__restrict__ stats,
                                                        uint32_t *__restrict__ err) {
     extern __shared__ __align__(128) uint8_t smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const int32_t words = (nbins + 31) / 32;
-    uint32_t *planes = reinterpret_cast<uint32_t *>(smem) + (size_t)warp * 3 * words;
-    uint16_t *list = reinterpret_cast<uint16_t *>(reinterpret_cast<uint32_t *>(smem) + (size_t)nw * 3 * words) +
-                     (size_t)warp * list_cap;
-    for (int32_t i = lane; i < 3 * words; i += 32) planes[i] = 0u;
+    const RankBufs rb = rank_bufs(smem + (size_t)warp * rank_bytes(nbins), nbins);
+    for (int32_t i = lane; i < (rb.words >> 1); i += 32) sts_u128(rb.pl + 16u * i, make_uint4(0u, 0u, 0u, 0u));
     __syncwarp();
-    const Planes pl{planes, planes + words, planes + 2 * words};
     const float mt_lane = db.mt[lane];
     float ma_lane = 0.0f;
 #pragma unroll
     for (int i = 0; i < kMaxMa; ++i)
         if (lane == i && i < mods.num_ma) ma_lane = mods.ma_mass[i];
-    const uint32_t total = min((uint32_t)*total_p, cap_iso);
+    const uint32_t total = wl.count(NC);
+    const uint32_t *work = wl.list(NC);
     // per-warp work counters (a warp's share of one launch fits 32 bits)
     uint32_t my_lists = 0, my_entries = 0, my_iso = 0, my_res = 0;
-    for (uint32_t t = blockIdx.x * nw + warp; t < total; t += gridDim.x * nw) {
+    for (uint32_t i = blockIdx.x * nw + warp; i < total; i += gridDim.x * nw) {
+        const uint32_t t = work[i];
         const uint64_t key = iso_key[t];
         const int32_t mu = (int32_t)((key >> 54) & 0x1FFu);
         const uint32_t p = (uint32_t)((key >> 27) & 0x7FFFFFFu);
-        if (key == ~0ull || p >= db.num_pep || mu >= mods.num_mod) {  // a skipped record
-            if (lane < kLevels) iso_len[(size_t)t * kLevels + lane] = 0;
-            continue;
-        }
         const uint32_t need = need_levels(cover, npep1, mu, p);
         const int zmax = 32 - __clz(need);
         const uint32_t tc = db.tc_sorted[p], tn = db.tn_sorted[p];
@@ -278,44 +288,21 @@ __global__ void __launch_bounds__(256) k_gen_iso_lists(DevDB db, DevMods mods, c
         }
         // the residues this isoform modifies (k_iso_positions)
         const ModPositions iso{iso_pos + (size_t)t * pos_words, ma_lane, 0u};
-        my_iso += 1;
-        my_res += tn > tc ? tn - tc : 0u;
         // mion_series.cu:226: residual + delta
         const float residual = __fadd_rn(db.r_sorted[p], mods.delta[mu]);
-        WordRange all{0x7FFFFFFF, 0};
-        // the level-z list from the planes, when some spectrum needs it
-        auto emit_level = [&](int z) {
-            if (!((need >> (z - 1)) & 1u)) return;
-            const WordRange use = all.hi > all.lo ? all : WordRange{0, 0};
-            uint16_t *slot = lists + off + (uint64_t)unit * (uint64_t)(z * (z - 1) / 2);
-            const int room = (int)(unit * (uint32_t)z);  // >= 10 (tn - tc) z distinct bins
-            int nl = compact_planes(pl, use, z == zmax, list, list_cap, slot, room);
-            if (nl > room) {
-                if (lane == 0) atomicOr(err, kErrListOverflow);
-                nl = room;
-            }
-            if (nl <= list_cap) {
-                const uint4 *src = reinterpret_cast<const uint4 *>(list);
-                uint4 *dst = reinterpret_cast<uint4 *>(slot);
-                for (int i = lane; i < ((nl + 7) >> 3); i += 32) dst[i] = src[i];
-            }
-            if (lane == 0) iso_len[(size_t)t * kLevels + (z - 1)] = (uint16_t)nl;
-            my_lists += 1;
-            my_entries += (uint32_t)nl;
-            __syncwarp();
-        };
-        auto widen = [&](WordRange wr) {
-            if (wr.hi > wr.lo) {
-                all.lo = min(all.lo, wr.lo);
-                all.hi = max(all.hi, wr.hi);
-            }
-        };
-        for (int z = 1; z <= zmax; ++z) {
-            widen(build_planes_range<FastDiv>(pl, db.ions, tc, tn, residual, z, z, nbins, mt_lane, iso));
-            emit_level(z);
+        // every level up to zmax has its place in the slot, unit z >= 10 (tn - tc) z entries
+        const ListSlots ls{lists + off, unit, 0ull, iso_len + (size_t)t * kLevels, 1ull};
+        const int entries = build_lists<FastDiv, NC>(rb, db.ions, tc, tn, residual, need, (uint32_t)nbins, mt_lane,
+                                                     iso, ls);
+        if (lane < kLevels && !((need >> lane) & 1u)) iso_len[(size_t)t * kLevels + lane] = 0;
+        if (entries < 0) {
+            if (lane == 0) wl.list(0)[atomicAdd(wl.w, 1u)] = t;
+            continue;
         }
-        if (lane >= zmax && lane < kLevels) iso_len[(size_t)t * kLevels + lane] = 0;
-        if (lane < zmax && !((need >> lane) & 1u)) iso_len[(size_t)t * kLevels + lane] = 0;
+        my_iso += 1u;
+        my_res += tn > tc ? tn - tc : 0u;
+        my_entries += (uint32_t)entries;
+        my_lists += (uint32_t)__popc(need);
     }
     if (stats && lane == 0) {
         atomicAdd(&stats[0], (unsigned long long)my_lists);
@@ -526,98 +513,11 @@ k_score_iso_lists(const uint16_t *__restrict__ lists, uint64_t list_total, const
     }
 }
 
-// ---- inclusive scan of 64-bit values (reduce, scan partials, apply) ----
-constexpr int kScan64Tile = 4096;
-
-__global__ void k_scan64_reduce(const unsigned long long *__restrict__ a, int64_t n,
-                                unsigned long long *__restrict__ partial) {
-    __shared__ unsigned long long red[32];
-    const int64_t base = (int64_t)blockIdx.x * kScan64Tile;
-    unsigned long long s = 0;
-    for (int i = threadIdx.x; i < kScan64Tile; i += blockDim.x)
-        if (base + i < n) s += a[base + i];
-    for (int o = 16; o >= 1; o >>= 1) s += __shfl_xor_sync(kFullMask, s, o);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        unsigned long long v = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0ull;
-        for (int o = 16; o >= 1; o >>= 1) v += __shfl_xor_sync(kFullMask, v, o);
-        if (threadIdx.x == 0) partial[blockIdx.x] = v;
-    }
-}
-
-__device__ __forceinline__ unsigned long long warp_incl_scan64(unsigned long long v) {
-    const int lane = threadIdx.x & 31;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const unsigned long long t = __shfl_up_sync(kFullMask, v, d);
-        if (lane >= d) v += t;
-    }
-    return v;
-}
-
-// single CTA: exclusive scan of the partials in place
-__global__ void k_scan64_partials(unsigned long long *__restrict__ partial, int64_t nb) {
-    __shared__ unsigned long long ws[32];
-    __shared__ unsigned long long carry;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
-    for (int64_t b0 = 0; b0 < nb; b0 += blockDim.x) {
-        const int64_t i = b0 + threadIdx.x;
-        const unsigned long long v = i < nb ? partial[i] : 0ull;
-        const unsigned long long x = warp_incl_scan64(v);
-        if (lane == 31) ws[warp] = x;
-        __syncthreads();
-        if (warp == 0) {
-            unsigned long long w = lane < (int)(blockDim.x >> 5) ? ws[lane] : 0ull;
-            w = warp_incl_scan64(w);
-            ws[lane] = w;
-        }
-        __syncthreads();
-        const unsigned long long before = carry + (warp ? ws[warp - 1] : 0ull);
-        if (i < nb) partial[i] = before + x - v;
-        __syncthreads();
-        if (threadIdx.x == blockDim.x - 1) carry = before + x;
-        __syncthreads();
-    }
-}
-
-__global__ void k_scan64_apply(const unsigned long long *__restrict__ a, int64_t n,
-                               const unsigned long long *__restrict__ partial, unsigned long long *__restrict__ out) {
-    __shared__ unsigned long long ws[32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int64_t base = (int64_t)blockIdx.x * kScan64Tile;
-    const int per = kScan64Tile / blockDim.x;
-    unsigned long long loc[16];
-    unsigned long long s = 0;
-    for (int k = 0; k < per; ++k) {
-        const int64_t i = base + (int64_t)threadIdx.x * per + k;
-        loc[k] = i < n ? a[i] : 0ull;
-        s += loc[k];
-    }
-    const unsigned long long x = warp_incl_scan64(s);
-    if (lane == 31) ws[warp] = x;
-    __syncthreads();
-    if (warp == 0) {
-        unsigned long long w = lane < (int)(blockDim.x >> 5) ? ws[lane] : 0ull;
-        w = warp_incl_scan64(w);
-        ws[lane] = w;
-    }
-    __syncthreads();
-    unsigned long long run = partial[blockIdx.x] + (warp ? ws[warp - 1] : 0ull) + x - s;
-    for (int k = 0; k < per; ++k) {
-        const int64_t i = base + (int64_t)threadIdx.x * per + k;
-        run += loc[k];
-        if (i < n) out[i] = run;
-    }
-}
-
 }  // namespace hfx
 
 using namespace hfx;
 
-int64_t hfx_iso_scan64_partials_needed(int64_t n) { return (n + kScan64Tile - 1) / kScan64Tile + 1; }
+int64_t hfx_iso_scan64_partials_needed(int64_t n) { return scan_partials<unsigned long long>(n); }
 
 int hfx_iso_plan(const DevDB &db, const DevMods &m, const SpecMeta *meta, int32_t nspec, const uint32_t *mb,
                  const uint32_t *me, const uint32_t *lstart, int32_t *cover, int32_t *cover_partial,
@@ -636,13 +536,7 @@ int hfx_iso_plan(const DevDB &db, const DevMods &m, const SpecMeta *meta, int32_
     k_iso_count<<<(unsigned)((n + 1 + 255) / 256), 256, 0, st>>>(db, m, cover, npep1, lstart, n, count, units);
     rc = hfx_scan_inclusive(count, n + 1, incl, count_partial, st);
     if (rc) return rc;
-    if (n > 0) {
-        const int64_t nb = (n + kScan64Tile - 1) / kScan64Tile;
-        k_scan64_reduce<<<(unsigned)nb, 512, 0, st>>>(units, n, units_partial);
-        k_scan64_partials<<<1, 1024, 0, st>>>(units_partial, nb);
-        k_scan64_apply<<<(unsigned)nb, 256, 0, st>>>(units, n, units_partial, incl_units);
-    }
-    return (int)cudaGetLastError();
+    return scan_inclusive<unsigned long long>(units, n, incl_units, units_partial, st);
 }
 
 int hfx_iso_expand(const DevDB &db, const DevMods &m, const int32_t *cover, const uint32_t *lstart,
@@ -659,28 +553,30 @@ int hfx_iso_expand(const DevDB &db, const DevMods &m, const int32_t *cover, cons
 
 int hfx_iso_generate(const DevDB &db, const DevMods &m, const int32_t *cover, int32_t nbins, const uint32_t *lstart,
                      const int32_t *total_p, uint32_t cap_iso, const uint64_t *iso_key, const uint64_t *iso_off,
-                     uint16_t *lists, uint64_t list_total, uint16_t *iso_len, int32_t list_cap, int32_t pos_words,
-                     uint32_t *iso_pos, int fastdiv, unsigned long long *stats, uint32_t *err, cudaStream_t st) {
+                     uint16_t *lists, uint64_t list_total, uint16_t *iso_len, int32_t pos_words,
+                     uint32_t *iso_pos, uint32_t *work, int fastdiv, unsigned long long *stats, uint32_t *err,
+                     cudaStream_t st) {
     if (cap_iso == 0) return 0;
     const int nw = 8;
-    const int32_t words = (nbins + 31) / 32;
-    // 16-byte staging lists of up to kStageCap entries (longer lists are
-    // written directly)
-    list_cap = (std::max(32, std::min(list_cap, kStageCap)) + 7) & ~7;
-    const size_t smem = (size_t)nw * 3 * words * 4 + (size_t)nw * list_cap * 2;
+    const size_t smem = (size_t)nw * rank_bytes(nbins);
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    k_iso_positions<<<(unsigned)((cap_iso + 255) / 256), 256, 0, st>>>(db, m, total_p, cap_iso, iso_key, pos_words,
-                                                                        iso_pos, err);
-    auto f = fastdiv ? k_gen_iso_lists<true> : k_gen_iso_lists<false>;
-    cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    int per = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, f, nw * 32, smem);
-    f<<<sms * (per > 0 ? per : 1), nw * 32, smem, st>>>(db, m, cover, (int64_t)db.num_pep + 1, nbins, lstart, total_p,
-                                                        cap_iso, iso_key, iso_off, lists, list_total, iso_len,
-                                                        list_cap, pos_words, iso_pos, stats, err);
+    const WorkLists wl{work, cap_iso};
+    cudaMemsetAsync(work, 0, 16, st);
+    k_iso_positions<<<(unsigned)(((uint64_t)cap_iso + 255) / 256), 256, 0, st>>>(
+        db, m, total_p, cap_iso, iso_key, pos_words, iso_pos, wl, iso_len, err);
+    auto run = [&](auto f, int most) {
+        cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        int per = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, f, nw * 32, smem);
+        f<<<sms * std::max(1, std::min(per, most)), nw * 32, smem, st>>>(
+            db, m, cover, (int64_t)db.num_pep + 1, nbins, lstart, iso_key, iso_off, lists, list_total, iso_len,
+            pos_words, iso_pos, wl, stats, err);
+    };
+    run(fastdiv ? k_gen_iso_lists<true, 1> : k_gen_iso_lists<false, 1>, 32);
+    run(fastdiv ? k_gen_iso_lists<true, 2> : k_gen_iso_lists<false, 2>, 32);
+    run(fastdiv ? k_gen_iso_lists<true, 0> : k_gen_iso_lists<false, 0>, 2);
     return (int)cudaGetLastError();
 }
 

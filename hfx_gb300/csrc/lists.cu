@@ -20,88 +20,12 @@
 #include "batched.h"
 #include "lists.h"
 #include "lists_device.cuh"
+#include "scan.cuh"
 #include <algorithm>
 #include <type_traits>
 #include "batched_common.cuh"
 
 namespace hfx {
-
-constexpr int kScanTile = 4096;
-
-// ---- multi-block inclusive scan of int32 (reduce, scan partials, apply) ----
-__global__ void k_scan_reduce(const int32_t *__restrict__ a, int64_t n, int32_t *__restrict__ partial) {
-    __shared__ int32_t red[32];
-    const int64_t base = (int64_t)blockIdx.x * kScanTile;
-    int32_t s = 0;
-    for (int i = threadIdx.x; i < kScanTile; i += blockDim.x)
-        if (base + i < n) s += a[base + i];
-    s = __reduce_add_sync(kFullMask, s);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        int32_t v = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0;
-        v = __reduce_add_sync(kFullMask, v);
-        if (threadIdx.x == 0) partial[blockIdx.x] = v;
-    }
-}
-
-__global__ void k_scan_partials(int32_t *__restrict__ partial, int32_t nb) {
-    // single CTA, exclusive scan in place
-    __shared__ int32_t ws[32];
-    __shared__ int32_t carry;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
-    for (int32_t b0 = 0; b0 < nb; b0 += blockDim.x) {
-        const int32_t i = b0 + threadIdx.x;
-        const int32_t v = i < nb ? partial[i] : 0;
-        const int32_t x = warp_incl_scan(v);
-        if (lane == 31) ws[warp] = x;
-        __syncthreads();
-        if (warp == 0) {
-            int32_t w = lane < (int)(blockDim.x >> 5) ? ws[lane] : 0;
-            w = warp_incl_scan(w);
-            ws[lane] = w;
-        }
-        __syncthreads();
-        const int32_t before = carry + (warp ? ws[warp - 1] : 0);
-        if (i < nb) partial[i] = before + x - v;
-        __syncthreads();
-        if (threadIdx.x == blockDim.x - 1) carry = before + x;
-        __syncthreads();
-    }
-}
-
-// Inclusive scan of one tile with its block offset: out[i] = sum a[0..i].
-__global__ void k_scan_apply(const int32_t *__restrict__ a, int64_t n, const int32_t *__restrict__ partial,
-                             int32_t *__restrict__ out) {
-    __shared__ int32_t ws[32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int64_t base = (int64_t)blockIdx.x * kScanTile;
-    const int per = kScanTile / blockDim.x;  // consecutive elements per thread
-    int32_t loc[16];
-    int32_t s = 0;
-    for (int k = 0; k < per; ++k) {
-        const int64_t i = base + (int64_t)threadIdx.x * per + k;
-        loc[k] = i < n ? a[i] : 0;
-        s += loc[k];
-    }
-    const int32_t x = warp_incl_scan(s);
-    if (lane == 31) ws[warp] = x;
-    __syncthreads();
-    if (warp == 0) {
-        int32_t w = lane < (int)(blockDim.x >> 5) ? ws[lane] : 0;
-        w = warp_incl_scan(w);
-        ws[lane] = w;
-    }
-    __syncthreads();
-    int32_t run = partial[blockIdx.x] + (warp ? ws[warp - 1] : 0) + x - s;
-    for (int k = 0; k < per; ++k) {
-        const int64_t i = base + (int64_t)threadIdx.x * per + k;
-        run += loc[k];
-        if (i < n) out[i] = run;
-    }
-}
 
 // ---- which (peptide, level) lists the batch needs ----
 __global__ void k_mark_levels(const SpecMeta *__restrict__ meta, const uint32_t *__restrict__ wb,
@@ -117,80 +41,72 @@ __global__ void k_mark_levels(const SpecMeta *__restrict__ meta, const uint32_t 
 }
 
 
-// One warp per candidate peptide: for every charge level some spectrum of
-// the batch needs, the sorted distinct-bin list, built incrementally (the
-// level-z planes are the level-(z-1) planes plus the charge-z ions).
-template <bool FastDiv>
-__global__ void __launch_bounds__(256) k_gen_lists(DevDB db, const int32_t *__restrict__ cover, int64_t npep1,
-                                                   int32_t nbins, const uint32_t *__restrict__ lstart,
-                                                   uint64_t total10, uint16_t *__restrict__ lists,
-                                                   uint16_t *__restrict__ list_len, int32_t list_cap,
-                                                   unsigned long long *__restrict__ stats,
-                                                   uint32_t *__restrict__ err) {
+// The candidates whose lists the batch needs, by class (entry: position |
+// levels << 27), and the lengths of the lists it does not need.  One thread
+// per peptide: a warp per peptide that looked at its coverage itself spent
+// 0.18 ms on the 1.4 M peptides of the 20,000-protein database however few
+// were needed.
+constexpr int kNeedShift = 27;  // positions are below 2^27
+__global__ void __launch_bounds__(256) k_list_work(DevDB db, const int32_t *__restrict__ cover, int64_t npep1,
+                                                   uint16_t *__restrict__ list_len, WorkLists wl) {
+    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+    int cls = -1;
+    uint32_t need = 0;
+    if (p < db.num_pep) {
+#pragma unroll
+        for (int z = 0; z < kLevels; ++z) {
+            if (cover[(int64_t)z * npep1 + p] > 0) need |= 1u << z;
+            else list_len[(size_t)z * db.num_pep + p] = 0;
+        }
+        if (need) cls = list_class(db.tc_sorted[p], db.tn_sorted[p]);
+    }
+    append_work(wl, cls, p | need << kNeedShift);
+}
+
+// One warp per needed candidate peptide of class NC: the sorted distinct-bin
+// list of every needed charge level (build_lists: the level-z list carries the
+// level-(z-1) list over and adds the charge-z ions).  The 3.84 M lists (946 M
+// entries) of 10,000 spectra against 20,000 proteins, coverage and work lists
+// included: 4.12 ms by bit planes and a bit loop, 2.51 ms by rank; issue 70 %
+// of the slots, shared memory 50 % of its wavefronts.
+template <bool FastDiv, int NC>
+__global__ void __launch_bounds__(256, NC == 0 ? 1 : 4) k_gen_lists(DevDB db, int32_t nbins,
+                                                                    const uint32_t *__restrict__ lstart,
+                                                                    uint64_t total10, uint16_t *__restrict__ lists,
+                                                                    uint16_t *__restrict__ list_len, WorkLists wl,
+                                                                    unsigned long long *__restrict__ stats) {
     extern __shared__ __align__(128) uint8_t smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const int32_t words = (nbins + 31) / 32;
-    uint32_t *planes = reinterpret_cast<uint32_t *>(smem) + (size_t)warp * 3 * words;
-    uint16_t *list = reinterpret_cast<uint16_t *>(reinterpret_cast<uint32_t *>(smem) + (size_t)nw * 3 * words) +
-                     (size_t)warp * list_cap;
+    const RankBufs rb = rank_bufs(smem + (size_t)warp * rank_bytes(nbins), nbins);
     __shared__ unsigned long long s_stats[3];
     if (threadIdx.x < 3) s_stats[threadIdx.x] = 0ull;
-    for (int32_t i = lane; i < 3 * words; i += 32) planes[i] = 0u;
+    for (int32_t i = lane; i < (rb.words >> 1); i += 32) sts_u128(rb.pl + 16u * i, make_uint4(0u, 0u, 0u, 0u));
     __syncthreads();
-    const Planes pl{planes, planes + words, planes + 2 * words};
     const float mt_lane = db.mt[lane];
-    unsigned long long my_lists = 0, my_entries = 0, my_res = 0;
-    for (int64_t t = (int64_t)blockIdx.x * nw + warp; t < (int64_t)db.num_pep; t += (int64_t)gridDim.x * nw) {
-        const uint32_t p = (uint32_t)t;
-        uint32_t need = 0;
-        if (lane < kLevels && cover[(int64_t)lane * npep1 + p] > 0) need = 1u;
-        need = __ballot_sync(kFullMask, need) & ((1u << kLevels) - 1u);
-        if (lane < kLevels && !((need >> lane) & 1u)) list_len[(size_t)lane * db.num_pep + p] = 0;
-        if (!need) continue;
-        const int zmax = 32 - __clz(need);
+    const uint32_t total = wl.count(NC);
+    const uint32_t *work = wl.list(NC);
+    uint32_t my_lists = 0, my_entries = 0, my_res = 0;
+    for (uint32_t t = blockIdx.x * nw + warp; t < total; t += gridDim.x * nw) {
+        const uint32_t w = work[t];
+        const uint32_t p = w & ((1u << kNeedShift) - 1u), need = w >> kNeedShift;
         const uint32_t tc = db.tc_sorted[p], tn = db.tn_sorted[p];
-        const float r = db.r_sorted[p];
-        my_res += tn > tc ? tn - tc : 0u;
-        WordRange all{0x7FFFFFFF, 0};
-        // the level-z list from the planes, when some spectrum needs it
-        auto emit_level = [&](int z) {
-            if (!((need >> (z - 1)) & 1u)) return;
-            const WordRange use = all.hi > all.lo ? all : WordRange{0, 0};
-            const uint64_t off = list_offset(lstart, total10, z, p);
-            const int room = (int)((lstart[p + 1] - lstart[p]) * (uint32_t)z);  // the slot, >= 10 (tn - tc) z
-            int n = compact_planes(pl, use, z == zmax, list, list_cap, lists + off, room);
-            if (n > room) {
-                if (lane == 0) atomicOr(err, kErrListOverflow);
-                n = room;
-            }
-            if (n <= list_cap) {
-                // 16-byte copies: the slot and the staging list start on
-                // 16-byte boundaries and hold n rounded up to 8 entries
-                const uint4 *src = reinterpret_cast<const uint4 *>(list);
-                uint4 *dst = reinterpret_cast<uint4 *>(lists + off);
-                for (int i = lane; i < ((n + 7) >> 3); i += 32) dst[i] = src[i];
-            }
-            if (lane == 0) list_len[(size_t)(z - 1) * db.num_pep + p] = (uint16_t)n;
-            my_lists += 1;
-            my_entries += (unsigned long long)n;
-            __syncwarp();
-        };
-        auto widen = [&](WordRange wr) {
-            if (wr.hi > wr.lo) {
-                all.lo = min(all.lo, wr.lo);
-                all.hi = max(all.hi, wr.hi);
-            }
-        };
-        for (int z = 1; z <= zmax; ++z) {
-            widen(build_planes_range<FastDiv>(pl, db.ions, tc, tn, r, z, z, nbins, mt_lane, NoMods{}));
-            emit_level(z);
+        // the slot holds 10 (tn - tc) z entries or more: every list fits
+        const ListSlots ls{lists, total10, lstart[p], list_len + p, db.num_pep};
+        const int entries = build_lists<FastDiv, NC>(rb, db.ions, tc, tn, db.r_sorted[p], need, (uint32_t)nbins,
+                                                     mt_lane, NoMods{}, ls);
+        if (entries < 0) {
+            if (lane == 0) wl.list(0)[atomicAdd(wl.w, 1u)] = w;
+            continue;
         }
+        my_entries += (uint32_t)entries;
+        my_lists += (uint32_t)__popc(need);
+        my_res += tn > tc ? tn - tc : 0u;
     }
     if (stats) {
         if (lane == 0) {
-            atomicAdd(&s_stats[0], my_lists);
-            atomicAdd(&s_stats[1], my_entries);
-            atomicAdd(&s_stats[2], my_res);
+            atomicAdd(&s_stats[0], (unsigned long long)my_lists);
+            atomicAdd(&s_stats[1], (unsigned long long)my_entries);
+            atomicAdd(&s_stats[2], (unsigned long long)my_res);
         }
         __syncthreads();
         if (threadIdx.x == 0) {
@@ -865,15 +781,10 @@ k_score_lists(const E *__restrict__ lists, const uint32_t *__restrict__ lstart, 
 using namespace hfx;
 
 int hfx_scan_inclusive(const int32_t *in, int64_t n, int32_t *out, int32_t *partial, cudaStream_t st) {
-    if (n <= 0) return 0;
-    const int64_t nb = (n + kScanTile - 1) / kScanTile;
-    k_scan_reduce<<<(unsigned)nb, 512, 0, st>>>(in, n, partial);
-    k_scan_partials<<<1, 1024, 0, st>>>(partial, (int32_t)nb);
-    k_scan_apply<<<(unsigned)nb, 256, 0, st>>>(in, n, partial, out);
-    return (int)cudaGetLastError();
+    return scan_inclusive<int32_t>(in, n, out, partial, st);
 }
 
-int64_t hfx_scan_partials_needed(int64_t n) { return (n + kScanTile - 1) / kScanTile + 1; }
+int64_t hfx_scan_partials_needed(int64_t n) { return scan_partials<int32_t>(n); }
 
 int hfx_lists_mark(const SpecMeta *meta, const uint32_t *wb, const uint32_t *we, int32_t nspec, int64_t npep1,
                    int32_t *diff, cudaStream_t st) {
@@ -882,25 +793,29 @@ int hfx_lists_mark(const SpecMeta *meta, const uint32_t *wb, const uint32_t *we,
     return (int)cudaGetLastError();
 }
 
+size_t hfx_lists_work_words(uint64_t n) { return work_words(n); }
+
 int hfx_lists_generate(const DevDB &db, const int32_t *cover, int64_t npep1, int32_t nbins, const uint32_t *lstart,
-                       uint64_t total10, uint16_t *lists, uint16_t *list_len, int32_t list_cap, int fastdiv,
-                       unsigned long long *stats, uint32_t *err, cudaStream_t st) {
+                       uint64_t total10, uint16_t *lists, uint16_t *list_len, uint32_t *work, int fastdiv,
+                       unsigned long long *stats, cudaStream_t st) {
     const int nw = 8;
-    const int32_t words = (nbins + 31) / 32;
-    // 16-byte staging lists of up to kStageCap entries (longer lists are
-    // written directly)
-    list_cap = (std::max(32, std::min(list_cap, kStageCap)) + 7) & ~7;
-    // per warp: three bit planes and a staging list of list_cap entries
-    const size_t smem = (size_t)nw * 3 * words * 4 + (size_t)nw * list_cap * 2;
+    const size_t smem = (size_t)nw * rank_bytes(nbins);
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    auto f = fastdiv ? k_gen_lists<true> : k_gen_lists<false>;
-    cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    int per = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, f, nw * 32, smem);
-    f<<<sms * (per > 0 ? per : 1), nw * 32, smem, st>>>(db, cover, npep1, nbins, lstart, total10, lists, list_len,
-                                                        list_cap, stats, err);
+    const WorkLists wl{work, db.num_pep};
+    cudaMemsetAsync(work, 0, 16, st);
+    k_list_work<<<(db.num_pep + 255) / 256, 256, 0, st>>>(db, cover, npep1, list_len, wl);
+    auto run = [&](auto f, int most) {
+        cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        int per = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, f, nw * 32, smem);
+        f<<<sms * std::max(1, std::min(per, most)), nw * 32, smem, st>>>(db, nbins, lstart, total10, lists, list_len,
+                                                                         wl, stats);
+    };
+    run(fastdiv ? k_gen_lists<true, 1> : k_gen_lists<false, 1>, 32);
+    run(fastdiv ? k_gen_lists<true, 2> : k_gen_lists<false, 2>, 32);
+    run(fastdiv ? k_gen_lists<true, 0> : k_gen_lists<false, 0>, 2);
     return (int)cudaGetLastError();
 }
 

@@ -5,7 +5,6 @@
 
 namespace hfx {
 constexpr int kLevels = 4;          // ion-charge levels 1..4 (Search.hs:182, ion_series.cu:301-309)
-constexpr int kMaxListLen = 4096;   // distinct bins kept per (peptide, level)
 }  // namespace hfx
 
 int hfx_scan_inclusive(const int32_t *in, int64_t n, int32_t *out, int32_t *partial, cudaStream_t st);
@@ -16,10 +15,12 @@ int hfx_lists_mark(const hfx::SpecMeta *meta, const uint32_t *wb, const uint32_t
 // over all peptides; the level-z list of p starts at
 // total10 * z(z-1)/2 + z * lstart[p].  stats (nullable, 8 counters): [0] lists
 // built, [1] list entries, [2] candidates scored, [3] entries streamed,
-// [4] peptide-spectrum pairs.
+// [4] peptide-spectrum pairs.  work: hfx_lists_work_words(num_pep) words of
+// scratch.
 int hfx_lists_generate(const hfx::DevDB &db, const int32_t *cover, int64_t npep1, int32_t nbins,
                        const uint32_t *lstart, uint64_t total10, uint16_t *lists, uint16_t *list_len,
-                       int32_t list_cap, int fastdiv, unsigned long long *stats, uint32_t *err, cudaStream_t st);
+                       uint32_t *work, int fastdiv, unsigned long long *stats, cudaStream_t st);
+size_t hfx_lists_work_words(uint64_t n);
 // Scorer over the lists; long_rows: 32-bit entries and group tiles read
 // from global memory (rows too long for shared memory), else 16-bit entries
 // and tiles staged in shared memory.
