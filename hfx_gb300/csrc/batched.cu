@@ -22,6 +22,7 @@
 #include "batched.h"
 #include "batched_common.cuh"
 #include "mods_device.cuh"
+#include "scan.cuh"
 #include <type_traits>
 
 namespace hfx {
@@ -49,41 +50,55 @@ __global__ void k_bucket_count(const SpecMeta *__restrict__ meta, int32_t nspec,
     atomicAdd(&hist[spec_bucket(m)], 1u);
 }
 
-// Single-CTA exclusive scan of n counters (in place), total in *total.
-__global__ void k_scan_u32(uint32_t *__restrict__ a, int32_t n, uint32_t *__restrict__ total) {
-    __shared__ uint32_t warp_sums[32];
-    __shared__ uint32_t carry;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (tid == 0) carry = 0;
-    __syncthreads();
-    for (int32_t base = 0; base < n; base += blockDim.x) {
-        const int32_t i = base + tid;
-        const uint32_t v = (i < n) ? a[i] : 0u;
-        uint32_t x = v;
+// Single-CTA exclusive scan of n counters (in place), total in *total.  A warp takes 512 neighbouring counters per round
+// in four 16-byte accesses a lane, so the 98,304 mass buckets take six rounds:
+// one counter per thread and round took 96, 45 us of a one-spectrum search.
+__global__ void __launch_bounds__(1024) k_scan_u32(uint32_t *__restrict__ a, int32_t n, uint32_t *__restrict__ total) {
+    __shared__ uint32_t ws[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t carry = 0;
+    const bool wide = on_16(a);
+    for (int64_t base = 0; base < n; base += 32 * kScanWarp<uint32_t>) {
+        const int64_t at = base + (int64_t)warp * kScanWarp<uint32_t>;
+        uint32_t v[kScanSteps][kScanVec<uint32_t>];
+        scan_load<uint32_t>(a, n, at, v);
+        uint32_t run = 0;
 #pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            uint32_t t = __shfl_up_sync(kFullMask, x, d);
-            if (lane >= d) x += t;
-        }
-        if (lane == 31) warp_sums[warp] = x;
-        __syncthreads();
-        if (warp == 0) {
-            uint32_t w = (lane < (int)(blockDim.x >> 5)) ? warp_sums[lane] : 0u;
+        for (int k = 0; k < kScanSteps; ++k) {
+            uint32_t own = 0;
 #pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                uint32_t t = __shfl_up_sync(kFullMask, w, d);
-                if (lane >= d) w += t;
+            for (int j = 0; j < 4; ++j) own += v[k][j];
+            const uint32_t x = warp_scan_of(own);
+            uint32_t e = run + x - own;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const uint32_t t = v[k][j];
+                v[k][j] = e;
+                e += t;
             }
-            warp_sums[lane] = w;
+            run += __shfl_sync(kFullMask, x, 31);
         }
+        if (lane == 0) ws[warp] = run;
         __syncthreads();
-        const uint32_t before = carry + (warp ? warp_sums[warp - 1] : 0u);
-        if (i < n) a[i] = before + x - v;
+        if (warp == 0) ws[lane] = warp_scan_of(ws[lane]);
         __syncthreads();
-        if (tid == blockDim.x - 1) carry = before + x;
+        const uint32_t before = carry + (warp ? ws[warp - 1] : 0u);
+        carry += ws[31];
+#pragma unroll
+        for (int k = 0; k < kScanSteps; ++k) {
+            const int64_t i = at + (int64_t)(k * 32 + lane) * 4;
+            if (wide && i + 4 <= n) {
+                *reinterpret_cast<uint4 *>(a + i) =
+                    make_uint4(before + v[k][0], before + v[k][1], before + v[k][2], before + v[k][3]);
+            } else {
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    if (i + j < n) a[i + j] = before + v[k][j];
+            }
+        }
         __syncthreads();
     }
-    if (tid == 0 && total) *total = carry;
+    if (threadIdx.x == 0 && total) *total = carry;
 }
 
 __global__ void k_bucket_scatter(const SpecMeta *__restrict__ meta, int32_t nspec, uint32_t *__restrict__ cursor,
@@ -96,20 +111,28 @@ __global__ void k_bucket_scatter(const SpecMeta *__restrict__ meta, int32_t nspe
     perm[pos] = s;
 }
 
+// With few_groups (no work-item size asked for) a group's window is cut so
+// that about this many items come of all groups together, four per resident
+// CTA of the list scorer: one spectrum's 3,400 candidates in one item kept one
+// SM busy for 0.22 ms.  From about 1,200 groups (76 of open windows) on the rule
+// changes nothing.
+constexpr uint32_t kFewItems = 1216;
+
 // One thread per group: members, union window, chunk count.
-// class_off[c] = first sorted position of class c (from the bucket scan).
-__global__ void k_groups(const uint32_t *__restrict__ bucket_off, const uint32_t *__restrict__ n_sorted,
+// bucket_end[b] = end of bucket b's spectra in sorted order (the scanned
+// counters, which the scatter has moved from the starts to the ends).
+__global__ void k_groups(const uint32_t *__restrict__ bucket_end, const uint32_t *__restrict__ n_sorted,
                          const int32_t *__restrict__ perm, const uint32_t *__restrict__ wb,
                          const uint32_t *__restrict__ we, const SpecMeta *__restrict__ meta, int32_t G,
-                         int32_t chunk, int32_t max_groups, GroupInfo *__restrict__ groups,
+                         int32_t chunk, int few_groups, int32_t max_groups, GroupInfo *__restrict__ groups,
                          uint32_t *__restrict__ nchunks, int32_t *__restrict__ group_of,
                          int32_t *__restrict__ slot_of, uint32_t *__restrict__ ngroups_out) {
     __shared__ uint32_t cls_start[kClasses + 1], grp_start[kClasses + 1];
     if (threadIdx.x == 0) {
         uint32_t gs = 0;
         for (int c = 0; c < kClasses; ++c) {
-            cls_start[c] = bucket_off[c * kMassBuckets];
-            const uint32_t end = (c + 1 < kClasses) ? bucket_off[(c + 1) * kMassBuckets] : *n_sorted;
+            cls_start[c] = c ? bucket_end[c * kMassBuckets - 1] : 0u;
+            const uint32_t end = bucket_end[(c + 1) * kMassBuckets - 1];
             grp_start[c] = gs;
             gs += (end - cls_start[c] + G - 1) / G;
         }
@@ -160,6 +183,10 @@ __global__ void k_groups(const uint32_t *__restrict__ bucket_off, const uint32_t
                        : (uint32_t)g >= ng - ng / 4 ? max(chunk / 4, 256)
                                                     : chunk;
     gi.chunk = group_chunk(gi.hi - gi.lo, cg);
+    if (few_groups) {
+        const uint64_t share = ((uint64_t)(gi.hi - gi.lo) * ng + kFewItems - 1) / kFewItems;
+        gi.chunk = (uint32_t)min((uint64_t)gi.chunk, max(share, (uint64_t)64));
+    }
     groups[g] = gi;
     nchunks[g] = (gi.hi - gi.lo + gi.chunk - 1) / gi.chunk;
 }
@@ -278,44 +305,16 @@ __global__ void k_merge_items(const float *__restrict__ part_s, const uint64_t *
     const int lane = threadIdx.x & 31;
     const int32_t s = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (s >= nspec) return;
-    typename std::conditional<R == 1, WarpTopK, WarpTopK64>::type tk;
+    typename std::conditional<R == 1, WarpList32, WarpList64>::type tk;
     tk.init();
     if (meta[s].status == 0) {
         const int32_t g = group_of[s], j = slot_of[s];
         for (uint32_t it = item_off[g]; it < item_off[g + 1]; ++it) {
             const size_t o = ((size_t)it * G + j) * K;
-            bool done = false;
-            for (int r = 0; r < R && !done; ++r) {
-                const int i = 32 * r + lane;
-                const float sc = i < K ? part_s[o + i] : -INFINITY;
-                const uint64_t kk = i < K ? part_k[o + i] : ~0ull;
-                for (int t = 0; t < 32 && 32 * r + t < K; ++t) {
-                    const float ts = __shfl_sync(kFullMask, sc, t);
-                    const uint64_t tk2 = __shfl_sync(kFullMask, kk, t);
-                    if (tk2 == ~0ull) {
-                        done = true;  // the item's list ends here
-                        break;
-                    }
-                    tk.insert(ts, tk2, kout);
-                }
-            }
+            tk.merge_list(part_s + o, part_k + o, K);
         }
     }
-    if constexpr (R == 1) {
-        if (lane < kout) {
-            out_s[(size_t)s * kout + lane] = tk.s;
-            out_k[(size_t)s * kout + lane] = tk.k;
-        }
-    } else {
-        if (lane < kout) {
-            out_s[(size_t)s * kout + lane] = tk.s0;
-            out_k[(size_t)s * kout + lane] = tk.k0;
-        }
-        if (32 + lane < kout) {
-            out_s[(size_t)s * kout + 32 + lane] = tk.s1;
-            out_k[(size_t)s * kout + 32 + lane] = tk.k1;
-        }
-    }
+    tk.store(out_s + (size_t)s * kout, out_k + (size_t)s * kout, kout);
 }
 
 // FP32 rescoring of the kept candidates (BF16/FP16-stored rows): one CTA
@@ -442,17 +441,16 @@ size_t hfx_batched_smem(int64_t stride, int elem_bytes, int G, int nw, int K) {
 }
 
 int hfx_batched_plan(const SpecMeta *meta, int32_t nspec, const uint32_t *wb, const uint32_t *we, int32_t G,
-                     int32_t chunk, const BatchedWs &ws, cudaStream_t st) {
+                     int32_t chunk, int few_groups, const BatchedWs &ws, cudaStream_t st) {
     const int nbk = kClasses * kMassBuckets;
     cudaMemsetAsync(ws.hist, 0, sizeof(uint32_t) * (nbk + 1), st);
     cudaMemsetAsync(ws.item_off, 0, sizeof(uint32_t) * (nspec + 1), st);
     k_bucket_count<<<(nspec + 255) / 256, 256, 0, st>>>(meta, nspec, ws.hist);
     k_scan_u32<<<1, 1024, 0, st>>>(ws.hist, nbk, ws.n_sorted);
-    cudaMemcpyAsync(ws.cursor, ws.hist, sizeof(uint32_t) * nbk, cudaMemcpyDeviceToDevice, st);
-    k_bucket_scatter<<<(nspec + 255) / 256, 256, 0, st>>>(meta, nspec, ws.cursor, ws.perm);
+    k_bucket_scatter<<<(nspec + 255) / 256, 256, 0, st>>>(meta, nspec, ws.hist, ws.perm);
     const int32_t max_groups = nspec;  // each class adds at most one partial group
     k_groups<<<(max_groups + 255) / 256, 256, 0, st>>>(ws.hist, ws.n_sorted, ws.perm, wb, we, meta, G, chunk,
-                                                       max_groups, ws.groups, ws.item_off, ws.group_of, ws.slot_of,
+                                                       few_groups, max_groups, ws.groups, ws.item_off, ws.group_of, ws.slot_of,
                                                        ws.ngroups);
     k_scan_u32<<<1, 1024, 0, st>>>(ws.item_off, max_groups + 1, ws.total_items);
     return (int)cudaGetLastError();

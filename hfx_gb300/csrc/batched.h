@@ -13,8 +13,7 @@ struct GroupInfo {
 };
 
 struct BatchedWs {
-    uint32_t *hist;         // [classes*buckets + 1] bucket counts -> offsets
-    uint32_t *cursor;       // [classes*buckets] scatter cursors
+    uint32_t *hist;         // [classes*buckets + 1] bucket counts -> starts -> ends (scatter cursors)
     uint32_t *n_sorted;     // [1] spectra placed
     int32_t *perm;          // [nspec] sorted position -> spectrum
     GroupInfo *groups;      // [nspec]
@@ -31,7 +30,7 @@ constexpr int kBucketCount = 12 * 8192;
 
 size_t hfx_batched_smem(int64_t stride, int elem_bytes, int G, int nw, int K);
 int hfx_batched_plan(const hfx::SpecMeta *meta, int32_t nspec, const uint32_t *wb, const uint32_t *we, int32_t G,
-                     int32_t chunk, const hfx::BatchedWs &ws, cudaStream_t st);
+                     int32_t chunk, int few_groups, const hfx::BatchedWs &ws, cudaStream_t st);
 // Runs the persistent scorer over the group tiles packed by hfx_pack_tiles
 // (tiles: ngroups * stride * G elements); nw = warps per CTA (0 = as many as shared memory holds,
 // at most 16), grid = CTAs (0 = one wave).

@@ -666,34 +666,99 @@ struct WarpTopK {
     }
 };
 
-// The same for up to 64 entries: lane l holds entries l (s0, k0) and
-// 32 + l (s1, k1).
-struct WarpTopK64 {
+// Compare-exchange with lane ^ d, the better entry to the lower lane.
+__device__ __forceinline__ void better_first(float &s, uint64_t &k, int d) {
+    const float os = __shfl_xor_sync(kFullMask, s, d);
+    const uint64_t ok = __shfl_xor_sync(kFullMask, k, d);
+    const bool lower = ((threadIdx.x & 31) & d) == 0;
+    if (better(os, ok, s, k) == lower) {
+        s = os;
+        k = ok;
+    }
+}
+
+// Merging whole sorted lists (best first, empty entries (-inf, ~0) last) into a
+// sorted warp list: the better of entry i of one and entry n - 1 - i of the
+// other are the best n of both as a bitonic sequence, which log2 n exchanges
+// sort.  About 60 instructions for 32 entries; inserting them one by one takes
+// 30 for each (0.22 ms for the 53 items of one spectrum's window).
+struct WarpList32 {
+    float s;
+    uint64_t k;
+    __device__ __forceinline__ void init() {
+        s = -INFINITY;
+        k = ~0ull;
+    }
+    __device__ __forceinline__ void merge(float os, uint64_t ok) {
+        const int lane = threadIdx.x & 31;
+        const float rs = __shfl_sync(kFullMask, os, 31 - lane);
+        const uint64_t rk = __shfl_sync(kFullMask, ok, 31 - lane);
+        if (better(rs, rk, s, k)) {
+            s = rs;
+            k = rk;
+        }
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) better_first(s, k, d);
+    }
+    // List `n` entries long at (ps, pk), n <= 32.
+    __device__ __forceinline__ void merge_list(const float *ps, const uint64_t *pk, int n) {
+        const int lane = threadIdx.x & 31;
+        merge(lane < n ? ps[lane] : -INFINITY, lane < n ? pk[lane] : ~0ull);
+    }
+    __device__ __forceinline__ void store(float *os, uint64_t *ok, int n) const {
+        const int lane = threadIdx.x & 31;
+        if (lane < n) {
+            os[lane] = s;
+            ok[lane] = k;
+        }
+    }
+};
+
+// Up to 64 entries: lane l holds entries l (s0, k0) and 32 + l (s1, k1).
+struct WarpList64 {
     float s0, s1;
     uint64_t k0, k1;
     __device__ __forceinline__ void init() {
         s0 = s1 = -INFINITY;
         k0 = k1 = ~0ull;
     }
-    __device__ __forceinline__ void insert(float ns, uint64_t nk, int K) {
+    __device__ __forceinline__ void merge_list(const float *ps, const uint64_t *pk, int n) {
         const int lane = threadIdx.x & 31;
-        const int i0 = lane, i1 = 32 + lane;
-        const uint32_t b0 = __ballot_sync(kFullMask, i0 < K && better(s0, k0, ns, nk));
-        const uint32_t b1 = __ballot_sync(kFullMask, i1 < K && better(s1, k1, ns, nk));
-        const int pos = __popc(b0) + __popc(b1);
-        // entry i moves to i + 1 for pos <= i < K - 1
-        const float u0 = __shfl_up_sync(kFullMask, s0, 1), u1 = __shfl_up_sync(kFullMask, s1, 1);
-        const uint64_t v0 = __shfl_up_sync(kFullMask, k0, 1), v1 = __shfl_up_sync(kFullMask, k1, 1);
-        const float c = __shfl_sync(kFullMask, s0, 31);  // entry 31 becomes entry 32
-        const uint64_t ck = __shfl_sync(kFullMask, k0, 31);
-        if (pos < K) {
-            if (i0 == pos) { s0 = ns; k0 = nk; }
-            else if (i0 > pos && i0 < K) { s0 = u0; k0 = v0; }
-            if (i1 == pos) { s1 = ns; k1 = nk; }
-            else if (i1 > pos && i1 < K) {
-                s1 = lane == 0 ? c : u1;
-                k1 = lane == 0 ? ck : v1;
-            }
+        // entries 63 - lane and 31 - lane of the other list
+        const int i1 = 63 - lane, i0 = 31 - lane;
+        const float a = i1 < n ? ps[i1] : -INFINITY, b = i0 < n ? ps[i0] : -INFINITY;
+        const uint64_t ka = i1 < n ? pk[i1] : ~0ull, kb = i0 < n ? pk[i0] : ~0ull;
+        if (better(a, ka, s0, k0)) {
+            s0 = a;
+            k0 = ka;
+        }
+        if (better(b, kb, s1, k1)) {
+            s1 = b;
+            k1 = kb;
+        }
+        if (better(s1, k1, s0, k0)) {
+            const float ts = s0;
+            const uint64_t tk = k0;
+            s0 = s1;
+            k0 = k1;
+            s1 = ts;
+            k1 = tk;
+        }
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) {
+            better_first(s0, k0, d);
+            better_first(s1, k1, d);
+        }
+    }
+    __device__ __forceinline__ void store(float *os, uint64_t *ok, int n) const {
+        const int lane = threadIdx.x & 31;
+        if (lane < n) {
+            os[lane] = s0;
+            ok[lane] = k0;
+        }
+        if (32 + lane < n) {
+            os[32 + lane] = s1;
+            ok[32 + lane] = k1;
         }
     }
 };

@@ -632,8 +632,6 @@ int32_t search_batched(hfx_ctx *ctx, const hfx_search_params *p, const Batch &b,
     BatchedWs ws;
     ws.hist = ctx->buf<uint32_t>("b_hist", kBucketCount + 1, e);
     if (e) return cuda_fail(ctx, e, "alloc");
-    ws.cursor = ctx->buf<uint32_t>("b_cursor", kBucketCount, e);
-    if (e) return cuda_fail(ctx, e, "alloc");
     uint32_t *scal = ctx->buf<uint32_t>("b_scal", 8, e);
     if (e) return cuda_fail(ctx, e, "alloc");
     ws.n_sorted = scal;
@@ -653,7 +651,7 @@ int32_t search_batched(hfx_ctx *ctx, const hfx_search_params *p, const Batch &b,
     ctx->stage_begin(HFX_STAGE_WINDOWS);
     int rc = hfx_launch_windows(ctx->d_r.as<float>(), (uint32_t)ctx->num_pep, meta, ns, wb, we, ctx->stream);
     if (rc) return cuda_fail(ctx, (cudaError_t)rc, "k_windows");
-    rc = hfx_batched_plan(meta, ns, wb, we, G, chunk, ws, ctx->stream);
+    rc = hfx_batched_plan(meta, ns, wb, we, G, chunk, p->chunk > 0 ? 0 : 1, ws, ctx->stream);
     if (rc) return cuda_fail(ctx, (cudaError_t)rc, "plan");
     ctx->stage_end(HFX_STAGE_WINDOWS, 6, ns);  // k_windows + 5 planning kernels
     uint32_t ngroups = 0, total_items = 0;
@@ -1531,7 +1529,6 @@ int32_t hfx_search_evalues(hfx_ctx *ctx, const hfx_search_params *p, const float
     // re-plan with FP32 groups of 4 over the search's workspace
     BatchedWs ws;
     ws.hist = ctx->buf<uint32_t>("b_hist", kBucketCount + 1, e);
-    ws.cursor = ctx->buf<uint32_t>("b_cursor", kBucketCount, e);
     uint32_t *scal = ctx->buf<uint32_t>("b_scal", 8, e);
     ws.n_sorted = scal;
     ws.ngroups = scal + 1;
@@ -1543,7 +1540,7 @@ int32_t hfx_search_evalues(hfx_ctx *ctx, const hfx_search_params *p, const float
     ws.group_of = ctx->buf<int32_t>("b_groupof", ns, e);
     ws.slot_of = ctx->buf<int32_t>("b_slotof", ns, e);
     if (e) return cuda_fail(ctx, e, "alloc");
-    rc = hfx_batched_plan(meta, ns, wb, we, G, chunk, ws, ctx->stream);
+    rc = hfx_batched_plan(meta, ns, wb, we, G, chunk, p->chunk > 0 ? 0 : 1, ws, ctx->stream);
     if (rc) return cuda_fail(ctx, (cudaError_t)rc, "plan");
     uint32_t hs[4];
     HFX_CUDA(cudaMemcpyAsync(hs, scal, 16, cudaMemcpyDeviceToHost, ctx->stream), "D2H plan");

@@ -247,7 +247,7 @@ __global__ void k_merge_with_mods(const float *__restrict__ ps, const uint64_t *
     const int lane = threadIdx.x & 31;
     const int32_t s = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (s >= nspec) return;
-    WarpTopK tk;
+    WarpList32 tk;
     tk.init();
     if (meta[s].status == 0) {
         const int32_t g = group_of[s], j = slot_of[s];
@@ -266,18 +266,11 @@ __global__ void k_merge_with_mods(const float *__restrict__ ps, const uint64_t *
             }
             for (uint32_t it = a; it < b; ++it) {
                 const size_t o = ((size_t)it * G + j) * K;
-                const float sc = lane < K ? sp[o + lane] : -INFINITY;
-                const uint64_t kk = lane < K ? kp[o + lane] : ~0ull;
-                const int nvalid = __popc(__ballot_sync(kFullMask, kk != ~0ull));
-                for (int t = 0; t < nvalid; ++t)
-                    tk.insert(__shfl_sync(kFullMask, sc, t), __shfl_sync(kFullMask, kk, t), K);
+                tk.merge_list(sp + o, kp + o, K);
             }
         }
     }
-    if (lane < K) {
-        out_s[(size_t)s * K + lane] = tk.s;
-        out_k[(size_t)s * K + lane] = tk.k;
-    }
+    tk.store(out_s + (size_t)s * K, out_k + (size_t)s * K, K);
 }
 
 // Isoform export for parity checks: for queries (mass-order position,

@@ -25,19 +25,20 @@ __device__ __forceinline__ uint32_t upper_bound_f(const float *a, uint32_t n, fl
     return lo;
 }
 
+// Two threads per spectrum: the even one searches the lower bound, the odd
+// one the upper, so the two chains of dependent loads run at once.
 __global__ void k_windows(const float *__restrict__ r_sorted, uint32_t n, const SpecMeta *__restrict__ meta,
                           int32_t nspec, uint32_t *__restrict__ wb, uint32_t *__restrict__ we) {
-    const int32_t s = blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int32_t s = (int32_t)(t >> 1);
+    const bool upper = t & 1;
+    uint32_t x = 0;
+    if (s < nspec && meta[s].status == 0)
+        x = upper ? upper_bound_f(r_sorted, n, meta[s].hi) : lower_bound_f(r_sorted, n, meta[s].lo);
+    const uint32_t b = __shfl_sync(kFullMask, x, (threadIdx.x & 31) & ~1);
     if (s >= nspec) return;
-    const SpecMeta m = meta[s];
-    uint32_t b = 0, e = 0;
-    if (m.status == 0) {
-        b = lower_bound_f(r_sorted, n, m.lo);
-        e = upper_bound_f(r_sorted, n, m.hi);
-        if (e < b) e = b;
-    }
-    wb[s] = b;
-    we[s] = e;
+    if (upper) we[s] = x < b ? b : x;
+    else wb[s] = x;
 }
 
 // Write every warp's list to shared memory and merge them in warp 0.
@@ -206,7 +207,7 @@ static size_t score_smem_bytes(int32_t len, int32_t words, int nw, int K) {
 int hfx_launch_windows(const float *r_sorted, uint32_t n, const SpecMeta *meta, int32_t nspec, uint32_t *wb,
                        uint32_t *we, cudaStream_t st) {
     if (nspec <= 0) return 0;
-    k_windows<<<(nspec + 127) / 128, 128, 0, st>>>(r_sorted, n, meta, nspec, wb, we);
+    k_windows<<<(unsigned)((2ll * nspec + 127) / 128), 128, 0, st>>>(r_sorted, n, meta, nspec, wb, we);
     return (int)cudaGetLastError();
 }
 
