@@ -732,7 +732,7 @@ int32_t search_batched(hfx_ctx *ctx, const hfx_search_params *p, const Batch &b,
         if (!rc) rc = hfx_scan_inclusive(diff, kLevels * npep1, cover, partial, ctx->stream);
         if (!rc && long_rows)
             rc = hfx_lists_generate_long(db, cover, npep1, (int32_t)stride, ctx->d_lstart.as<uint32_t>(), total10,
-                                         (uint32_t *)lists, llen, p->fastdiv,
+                                         (uint32_t *)lists, llen, work, p->fastdiv,
                                          p->ion_bins_custom ? p->bin_width : 0.0f, stats,
                                          ctx->d_err.as<uint32_t>(), ctx->stream);
         else if (!rc)
@@ -740,7 +740,7 @@ int32_t search_batched(hfx_ctx *ctx, const hfx_search_params *p, const Batch &b,
                                     ctx->d_lstart.as<uint32_t>(), total10, (uint16_t *)lists, llen, work,
                                     p->fastdiv, stats, ctx->stream);
         if (rc) return cuda_fail(ctx, (cudaError_t)rc, "ion lists");
-        ctx->stage_end(HFX_STAGE_LISTS, long_rows ? 5 : 8, 0);
+        ctx->stage_end(HFX_STAGE_LISTS, 8, 0);  // mark, 3 scans, k_list_work, 3 classes of k_gen_lists
         ctx->stage_begin(HFX_STAGE_SCORE);
         float *sink = nullptr;
         const uint64_t *sink_off = nullptr;

@@ -47,8 +47,11 @@ __global__ void k_mark_levels(const SpecMeta *__restrict__ meta, const uint32_t 
 // 0.18 ms on the 1.4 M peptides of the 20,000-protein database however few
 // were needed.
 constexpr int kNeedShift = 27;  // positions are below 2^27
+__device__ __forceinline__ int long_class(uint32_t tc, uint32_t tn, uint32_t need);
+template <bool kLong>
 __global__ void __launch_bounds__(256) k_list_work(DevDB db, const int32_t *__restrict__ cover, int64_t npep1,
-                                                   uint16_t *__restrict__ list_len, WorkLists wl) {
+                                                   uint16_t *__restrict__ list_len, WorkLists wl,
+                                                   uint32_t *__restrict__ err) {
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
     int cls = -1;
     uint32_t need = 0;
@@ -58,7 +61,14 @@ __global__ void __launch_bounds__(256) k_list_work(DevDB db, const int32_t *__re
             if (cover[(int64_t)z * npep1 + p] > 0) need |= 1u << z;
             else list_len[(size_t)z * db.num_pep + p] = 0;
         }
-        if (need) cls = list_class(db.tc_sorted[p], db.tn_sorted[p]);
+        if (need) {
+            const uint32_t tc = db.tc_sorted[p], tn = db.tn_sorted[p];
+            cls = kLong ? long_class(tc, tn, need) : list_class(tc, tn);
+            if (cls < 0) {  // more keys than a warp sorts
+                atomicOr(err, kErrTooLong);
+                for (int z = 0; z < kLevels; ++z) list_len[(size_t)z * db.num_pep + p] = 0;
+            }
+        }
     }
     append_work(wl, cls, p | need << kNeedShift);
 }
@@ -119,262 +129,186 @@ __global__ void __launch_bounds__(256, NC == 0 ? 1 : 4) k_gen_lists(DevDB db, in
 
 // ---- long rows: 32-bit list entries built by sorting ----
 //
-// With ~10^5 bins per row the three bit planes no longer fit in shared
-// memory.  Instead, for every needed (peptide, level z) the warp writes the
-// ten keys (bin << 2 | level) of every (prefix, charge 1..z) into a per-warp
-// buffer (ion_series.cu:78-123, the same arithmetic as emit_ions), sorts the
-// buffer, and keeps the last key of each bin, i.e. its highest level -- the
-// reference's atomicMax into the dense row (ion_series.cu:71-75).
-constexpr int kLongKeys = 4096;  // keys per warp: 32-prefix chunks x charges x 10
+// With ~10^5 bins per row a bit per bin no longer fits in shared memory.
+// Instead the warp writes the ten keys (bin, charge, level) of every (prefix,
+// charge 1..zmax) of a needed peptide (ion_series.cu:78-123, the same
+// arithmetic as item_bits) and sorts them once: a counting sort into up to 512
+// ranges of bins (shared-memory counters, one scan, one scatter), then each
+// key's place among the few keys of its range by comparing with them.  A key
+// that opens a bin's run reads the run and has, for every charge level, the
+// bin's highest level among the charges up to it -- the reference's atomicMax
+// into the dense row (ion_series.cu:71-75) -- and ballots place it in the
+// lists of the needed levels.
+//
+// What bounds it: shared-memory latency and instruction issue.  A bitonic sort
+// per level with eight warps an SM (128 KB of keys) took 130 ms for the 4.2 M
+// lists of a 10,000-spectrum batch at 0.02 Da; this takes 10.3 ms.
+constexpr int kLongKeys = 4096;      // keys of a peptide that is accepted
+constexpr int kLongRanges = 512;     // counting-sort ranges
 
-// rint(mz / width): the mono width as in bin_of, or a custom ion width
-// (ibw > 0, the 0.02 Da switch) by IEEE division (__fdividef with FastDiv).
-template <bool FastDiv>
-__device__ __forceinline__ int32_t bin_w(float mz, float ibw) {
-    if (ibw > 0.0f) return sat_bin(rintf(FastDiv ? __fdividef(mz, ibw) : __fdiv_rn(mz, ibw)));
-    return bin_of<FastDiv>(mz);
+// Class of a peptide by its keys: 1, 2 and 0 hold up to 1,024, 2,048 and
+// kLongKeys keys (9, 18 and 34 KB of shared memory a warp); -1: too long.
+__host__ __device__ constexpr int long_keys(int cls) { return cls == 1 ? 1024 : (cls == 2 ? 2048 : kLongKeys); }
+__device__ __forceinline__ int long_class(uint32_t tc, uint32_t tn, uint32_t need) {
+    if (tn < tc) return -1;
+    const uint64_t n = 10ull * (tn - tc) * (uint32_t)(32 - __clz(need));
+    return n <= 1024u ? 1 : (n <= 2048u ? 2 : (n <= (uint64_t)kLongKeys ? 0 : -1));
+}
+__host__ __device__ constexpr size_t long_bytes(int cls) { return (size_t)long_keys(cls) * 8 + kLongRanges * 4; }
+
+// The bin rint(mz / d), y = RN(1 / d), for the mono or a custom width; from
+// 2^22 on -- beyond every row -- the uncorrected product, which keeps the
+// conversion's saturation.
+__device__ __forceinline__ uint32_t bin_long(float mz, float d, float y) {
+    const float q = __fmul_rn(mz, y);
+    return __float2uint_rz(q < 4194304.0f ? rintf(quotient(mz, d, y)) : q);
 }
 
-template <bool FastDiv>
-__device__ __forceinline__ void emit_keys(float b, float y, const ChargeConst &k, int32_t nbins, float ibw,
-                                          uint32_t *out) {
-    auto key = [&](int32_t x, uint32_t lvl) -> uint32_t {
-        return (x >= 0 && x < nbins) ? (((uint32_t)x << 2) | lvl) : 0xFFFFFFFFu;
-    };
-    // A ion
-    out[0] = key(bin_w<FastDiv>(div_charge<FastDiv>(__fadd_rn(__fsub_rn(b, kCO), k.hc), k.c), ibw), 1u);
-    // B ions: x-1, x, x+1 at 25/50/25, and the water and ammonia losses at 10
-    float m = div_charge<FastDiv>(__fadd_rn(b, k.hc), k.c);
-    int32_t x = bin_w<FastDiv>(m, ibw);
-    out[1] = key(x - 1, 2u);
-    out[2] = key(x, 3u);
-    out[3] = key(x + 1, 2u);
-    out[4] = key(bin_w<FastDiv>(__fsub_rn(m, k.dh2o), ibw), 1u);
-    out[5] = key(bin_w<FastDiv>(__fsub_rn(m, k.dnh3), ibw), 1u);
-    // Y ions
-    m = div_charge<FastDiv>(__fadd_rn(__fadd_rn(y, kH2O), k.hc), k.c);
-    x = bin_w<FastDiv>(m, ibw);
-    out[6] = key(x - 1, 2u);
-    out[7] = key(x, 3u);
-    out[8] = key(x + 1, 2u);
-    out[9] = key(bin_w<FastDiv>(__fsub_rn(m, k.dnh3), ibw), 1u);
-}
-
-// Warp-wide bitonic sort of n2 (a power of two) keys in shared memory,
-// ascending (or descending).
-__device__ __forceinline__ void warp_bitonic_sort(uint32_t *kb, int32_t n2, bool descending = false) {
-    const int lane = threadIdx.x & 31;
-    for (int32_t kk = 2; kk <= n2; kk <<= 1) {
-        for (int32_t j = kk >> 1; j > 0; j >>= 1) {
-            for (int32_t i = lane; i < n2; i += 32) {
-                const int32_t l = i ^ j;
-                if (l > i) {
-                    const uint32_t a = kb[i], b = kb[l];
-                    if ((a > b) == (((i & kk) == 0) != descending)) {
-                        kb[i] = b;
-                        kb[l] = a;
-                    }
-                }
-            }
-            __syncwarp();
-        }
-    }
-}
-
-// Ascending bitonic merge of n2 keys whose first half ascends and second
-// half descends.
-__device__ __forceinline__ void warp_bitonic_merge(uint32_t *kb, int32_t n2) {
-    const int lane = threadIdx.x & 31;
-    for (int32_t j = n2 >> 1; j > 0; j >>= 1) {
-        for (int32_t i = lane; i < n2; i += 32) {
-            const int32_t l = i ^ j;
-            if (l > i) {
-                const uint32_t a = kb[i], b = kb[l];
-                if (a > b) {
-                    kb[i] = b;
-                    kb[l] = a;
-                }
-            }
-        }
-        __syncwarp();
-    }
-}
-
-// Keeps the last key of each bin (its highest level) of the ascending keys
-// kb[0, n2), packed in order at kb[0, n) (in place: a round reads its keys
-// before it writes, and writes only at or below them), and, when out is
-// given, at out[0, min(n, cap)).  Returns n.
-__device__ __forceinline__ int32_t warp_keep_highest(uint32_t *kb, int32_t n2, uint32_t *out, int32_t cap) {
-    const int lane = threadIdx.x & 31;
-    int32_t n = 0;
-    for (int32_t i0 = 0; i0 < n2; i0 += 32) {
-        const int32_t i = i0 + lane;
-        const uint32_t k = i < n2 ? kb[i] : 0xFFFFFFFFu;
-        const bool keep = k != 0xFFFFFFFFu && (i + 1 >= n2 || (kb[i + 1] >> 2) != (k >> 2));
-        const uint32_t bal = __ballot_sync(kFullMask, keep);
-        const int32_t at = n + __popc(bal & ((1u << lane) - 1u));
-        if (keep) {
-            kb[at] = k;
-            if (out && at < cap) out[at] = k;
-        }
-        n += __popc(bal);
-    }
-    __syncwarp();
-    return n;
-}
-
-template <bool FastDiv>
-__global__ void __launch_bounds__(256) k_gen_lists_long(DevDB db, const int32_t *__restrict__ cover, int64_t npep1,
-                                                        int32_t nbins, const uint32_t *__restrict__ lstart,
+template <bool FastDiv, int kClass>
+__global__ void __launch_bounds__(256) k_gen_lists_long(DevDB db, int32_t nbins, const uint32_t *__restrict__ lstart,
                                                         uint64_t total10, uint32_t *__restrict__ lists,
-                                                        uint16_t *__restrict__ list_len, float ibw,
-                                                        unsigned long long *__restrict__ stats,
-                                                        uint32_t *__restrict__ err) {
-    extern __shared__ __align__(16) uint32_t keybuf[];
+                                                        uint16_t *__restrict__ list_len, float width, WorkLists wl,
+                                                        unsigned long long *__restrict__ stats) {
+    extern __shared__ __align__(16) uint8_t smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    uint32_t *kb = keybuf + (size_t)warp * kLongKeys;
+    const uint32_t ka = smem_u32(smem) + (uint32_t)warp * (uint32_t)long_bytes(kClass);
+    const uint32_t kb = ka + (uint32_t)long_keys(kClass) * 4u, cnt = kb + (uint32_t)long_keys(kClass) * 4u;
     __shared__ unsigned long long s_stats[3];
     if (threadIdx.x < 3) s_stats[threadIdx.x] = 0ull;
     __syncthreads();
     const float mt_lane = db.mt[lane];
+    const float rwidth = __fdiv_rn(1.0f, width);
+    // ranges of 2^shift bins
+    int shift = 0;
+    while ((nbins >> shift) >= kLongRanges) ++shift;
+    const uint32_t total = wl.count(kClass);
+    const uint32_t *work = wl.list(kClass);
     uint32_t my_lists = 0, my_entries = 0, my_res = 0;
-    for (int64_t t = (int64_t)blockIdx.x * nw + warp; t < (int64_t)db.num_pep; t += (int64_t)gridDim.x * nw) {
-        const uint32_t p = (uint32_t)t;
-        uint32_t need = 0;
-        if (lane < kLevels && cover[(int64_t)lane * npep1 + p] > 0) need = 1u;
-        need = __ballot_sync(kFullMask, need) & ((1u << kLevels) - 1u);
-        if (lane < kLevels && !((need >> lane) & 1u)) list_len[(size_t)lane * db.num_pep + p] = 0;
-        if (!need) continue;
+    for (uint32_t t = blockIdx.x * nw + warp; t < total; t += gridDim.x * nw) {
+        const uint32_t p = work[t] & ((1u << kNeedShift) - 1u), need = work[t] >> kNeedShift;
         const int zmax = 32 - __clz(need);
-        const uint32_t tc = db.tc_sorted[p], tn = db.tn_sorted[p];
-        const float r = db.r_sorted[p];
-        my_res += tn > tc ? tn - tc : 0u;
-        const uint32_t nchunk = (tn - tc + 31u) / 32u;
-        // keys of (prefix k, charge c) at 10 (k z + c - 1), padded to a power of two
-        uint32_t nmax = 32u;
-        while (tn >= tc && nmax < (tn - tc) * (uint32_t)zmax * 10u) nmax <<= 1;
-        if (tn < tc || nmax > (uint32_t)kLongKeys) {
-            if (lane == 0) atomicOr(err, kErrTooLong);
-            if (lane < kLevels && ((need >> lane) & 1u)) list_len[(size_t)lane * db.num_pep + p] = 0;
-            continue;
-        }
-        // Incremental levels where they fit: the level-z list is the
-        // level-(z-1) list (ascending, in the lower half) merged with the
-        // sorted charge-z keys (descending, in the upper half) by one bitonic
-        // merge, then reduced to each bin's highest level -- the same list as
-        // sorting every charge <= z at once, with a tenth of the
-        // compare-exchanges.  A peptide whose lists outgrow half the buffer
-        // takes the full sort below.
-        const int32_t nk = 10 * (int32_t)(tn - tc);  // keys of one charge
-        int32_t hmax = 32;
-        while (hmax < max(nk, nk * (zmax - 1))) hmax <<= 1;
-        if (2 * hmax <= kLongKeys) {
-            int32_t n_prev = 0;
+        const uint32_t tc = db.tc_sorted[p];
+        const int len = (int)(db.tn_sorted[p] - tc);
+        const float residual = db.r_sorted[p];
+        const uint32_t slot = lstart[p];
+        my_res += (uint32_t)len;
+#pragma unroll
+        for (int i = 0; i < kLongRanges / 128; ++i) sts_u128(cnt + 16u * (uint32_t)(32 * i + lane), make_uint4(0u, 0u, 0u, 0u));
+        __syncwarp();
+        // the keys bin << 4 | (charge - 1) << 2 | level (~0: outside the row),
+        // charge by charge, and how many fall into each range
+        float carry = 0.0f;
+        for (int k0 = 0; k0 < len; k0 += 32) {
+            NoMods mods;
+            const int c32 = min(32, len - k0);
+            const float b = ladder_chunk(db.ions, tc + (uint32_t)k0, c32, mt_lane, mods, carry);
+            carry = __shfl_sync(kFullMask, b, c32 - 1);
+            const float y = __fsub_rn(residual, b);
+#pragma unroll 1
             for (int z = 1; z <= zmax; ++z) {
-                int32_t h = 32;
-                while (h < max(nk, n_prev)) h <<= 1;
-                const int32_t lo = z == 1 ? 0 : h;  // where the charge-z keys go
-                const int32_t n2 = z == 1 ? h : 2 * h;
-                for (int32_t i = n_prev + lane; i < n2; i += 32) kb[i] = 0xFFFFFFFFu;
-                __syncwarp();
-                float carry = 0.0f;
-                for (uint32_t ci = 0; ci < nchunk; ++ci) {
-                    const uint32_t base = tc + 32u * ci;
-                    const int cnt = (int)min(32u, tn - base);
-                    uint32_t byte = 0;
-                    if (lane < cnt) byte = __ldg(db.ions + base + lane);
-                    float v = residue_mass(mt_lane, byte);
-                    if (lane >= cnt) v = 0.0f;
-                    if (lane == 0) v = __fadd_rn(v, carry);
+                const ChargeConst kc = charge_const<FastDiv>(z);
+                auto bin = [&](float mz) -> uint32_t {
+                    if constexpr (FastDiv) return (uint32_t)sat_bin(rintf(__fdividef(mz, width)));
+                    else return bin_long(mz, width, rwidth);
+                };
+                const float mb = div_charge<FastDiv>(__fadd_rn(b, kc.hc), z);
+                const float my = div_charge<FastDiv>(__fadd_rn(__fadd_rn(y, kH2O), kc.hc), z);
+                const uint32_t xb = bin(mb), xy = bin(my);
+                const uint32_t x[10] = {bin(div_charge<FastDiv>(__fadd_rn(__fsub_rn(b, kCO), kc.hc), z)),
+                                        bin(__fsub_rn(mb, kc.dh2o)),
+                                        bin(__fsub_rn(mb, kc.dnh3)),
+                                        bin(__fsub_rn(my, kc.dnh3)),
+                                        xb - 1u, xb + 1u, xy - 1u, xy + 1u, xb, xy};
+                const uint32_t at = ka + 40u * (uint32_t)((z - 1) * len + k0 + lane);
+                if (lane < c32) {
 #pragma unroll
-                    for (int d = 1; d < 32; d <<= 1) {
-                        const float u = __shfl_up_sync(kFullMask, v, d);
-                        if (lane >= d) v = __fadd_rn(v, u);
+                    for (int j = 0; j < 10; ++j) {
+                        const bool in = x[j] < (uint32_t)nbins;
+                        const uint32_t key = x[j] << 4 | (uint32_t)(z - 1) << 2 | (j < 4 ? 1u : (j < 8 ? 2u : 3u));
+                        sts_u32(at + 4u * j, in ? key : ~0u);
+                        if (in) red_add(cnt + 4u * (x[j] >> shift), 1u);
                     }
-                    carry = __shfl_sync(kFullMask, v, cnt - 1);
-                    if (lane < cnt)
-                        emit_keys<FastDiv>(v, __fsub_rn(r, v), charge_const<FastDiv>(z), nbins, ibw,
-                                           kb + lo + (size_t)(32u * ci + (uint32_t)lane) * 10);
                 }
-                __syncwarp();
-                if (z == 1) {
-                    warp_bitonic_sort(kb, n2);
-                } else {
-                    warp_bitonic_sort(kb + h, h, true);
-                    warp_bitonic_merge(kb, n2);
-                }
-                const bool needed = (need >> (z - 1)) & 1u;
-                const int32_t slot = 10 * z * (int32_t)(tn - tc);
-                int32_t n = warp_keep_highest(kb, n2, needed ? lists + list_offset(lstart, total10, z, p) : nullptr,
-                                              slot);
-                n_prev = n;
-                if (!needed) continue;
-                if (n > slot) {
-                    if (lane == 0) atomicOr(err, kErrListOverflow);
-                    n = slot;
-                }
-                if (lane == 0) list_len[(size_t)(z - 1) * db.num_pep + p] = (uint16_t)min(n, 65535);
-                my_lists += 1u;
-                my_entries += (uint32_t)n;
-                __syncwarp();
             }
-            continue;
         }
-        for (int z = 1; z <= zmax; ++z) {
-            if (!((need >> (z - 1)) & 1u)) continue;
-            const int32_t nslot = (int32_t)(tn - tc) * z * 10;
-            int32_t n2 = 32;
-            while (n2 < nslot) n2 <<= 1;
-            for (int32_t i = lane; i < n2; i += 32) kb[i] = 0xFFFFFFFFu;
-            __syncwarp();
-            // the b-ladder: the reference warp scan per 32-residue chunk
-            float carry = 0.0f;
-            for (uint32_t ci = 0; ci < nchunk; ++ci) {
-                const uint32_t base = tc + 32u * ci;
-                const int cnt = (int)min(32u, tn - base);
-                uint32_t byte = 0;
-                if (lane < cnt) byte = __ldg(db.ions + base + lane);
-                float v = residue_mass(mt_lane, byte);
-                if (lane >= cnt) v = 0.0f;
-                if (lane == 0) v = __fadd_rn(v, carry);
+        __syncwarp();
+        // starts of the ranges
+        uint32_t n = 0;
+#pragma unroll 1
+        for (int i = 0; i < kLongRanges / 128; ++i) {
+            const uint32_t at = cnt + 16u * (uint32_t)(32 * i + lane);
+            const uint4 c = lds_u128(at);
+            const uint32_t own = c.x + c.y + c.z + c.w;
+            const uint32_t incl = (uint32_t)warp_incl_scan((int)own);
+            const uint32_t e = n + incl - own;
+            sts_u128(at, make_uint4(e, e + c.x, e + c.x + c.y, e + c.x + c.y + c.z));
+            n += __shfl_sync(kFullMask, incl, 31);
+        }
+        __syncwarp();
+        // scatter; a range's counter ends at its end
+        const int raw = 10 * len * zmax;
+#pragma unroll 1
+        for (int i = lane; i < raw; i += 32) {
+            const uint32_t k = lds_u32(ka + 4u * i);
+            if (k != ~0u) sts_u32(kb + 4u * atom_add(cnt + 4u * (k >> (4 + shift)), 1u), k);
+        }
+        __syncwarp();
+        // each key's place within its range
+#pragma unroll 1
+        for (int i = lane; i < (int)n; i += 32) {
+            const uint32_t k = lds_u32(kb + 4u * i);
+            const uint32_t r = k >> (4 + shift);
+            uint32_t at = r ? lds_u32(cnt + 4u * r - 4u) : 0u;
+            const uint32_t end = lds_u32(cnt + 4u * r);
+            uint32_t place = at;
+            for (; at < end; ++at) {
+                const uint32_t o = lds_u32(kb + 4u * at);
+                place += (o < k || (o == k && at < (uint32_t)i)) ? 1u : 0u;
+            }
+            sts_u32(ka + 4u * place, k);
+        }
+        __syncwarp();
+        // the runs of equal bins; byte z - 1 of `best`: the highest level up to charge z
+        uint32_t out_n[kLevels];
 #pragma unroll
-                for (int d = 1; d < 32; d <<= 1) {
-                    const float u = __shfl_up_sync(kFullMask, v, d);
-                    if (lane >= d) v = __fadd_rn(v, u);
+        for (int z = 0; z < kLevels; ++z) out_n[z] = 0u;
+#pragma unroll 1
+        for (int i0 = 0; i0 < (int)n; i0 += 32) {
+            const int i = i0 + lane;
+            uint32_t best = 0u, bin = ~0u;
+            if (i < (int)n) {
+                const uint32_t k = lds_u32(ka + 4u * i);
+                bin = k >> 4;
+                if (i == 0 || (lds_u32(ka + 4u * i - 4u) >> 4) != bin) {
+                    uint32_t o = k;
+                    for (int j = i;;) {
+                        const uint32_t c = (o >> 2) & 3u;
+                        best = __vmaxu4(best, ((o & 3u) * 0x01010101u) << (8u * c));
+                        if (++j >= (int)n) break;
+                        o = lds_u32(ka + 4u * j);
+                        if ((o >> 4) != bin) break;
+                    }
                 }
-                carry = __shfl_sync(kFullMask, v, cnt - 1);
-                if (lane < cnt) {
-                    const float y = __fsub_rn(r, v);
-                    const uint32_t k = 32u * ci + (uint32_t)lane;
-                    for (int c = 1; c <= z; ++c)
-                        emit_keys<FastDiv>(v, y, charge_const<FastDiv>(c), nbins, ibw,
-                                           kb + ((size_t)k * z + (c - 1)) * 10);
-                }
             }
-            __syncwarp();
-            warp_bitonic_sort(kb, n2);
-            // keep the last key of each bin (its highest level), in order
-            const uint64_t off = list_offset(lstart, total10, z, p);
-            const int32_t slot = 10 * z * (int32_t)(tn - tc);
-            int32_t n = 0;
-            for (int32_t i0 = 0; i0 < n2; i0 += 32) {
-                const int32_t i = i0 + lane;
-                const uint32_t k = kb[i];
-                const bool keep = k != 0xFFFFFFFFu && (i + 1 == n2 || (kb[i + 1] >> 2) != (k >> 2));
-                const uint32_t bal = __ballot_sync(kFullMask, keep);
-                const int32_t at = n + __popc(bal & ((1u << lane) - 1u));
-                if (keep && at < slot) lists[off + at] = k;
-                n += __popc(bal);
+#pragma unroll
+            for (int z = 0; z < kLevels; ++z) {
+                if (!((need >> z) & 1u)) continue;
+                const uint32_t lvl = (best >> (8 * z)) & 0xFFu;
+                const uint32_t bal = __ballot_sync(kFullMask, lvl != 0u);
+                if (lvl)
+                    lists[total10 * (uint64_t)(z * (z + 1) / 2) + (uint64_t)(z + 1) * slot + out_n[z] +
+                          (uint32_t)__popc(bal & ((1u << lane) - 1u))] = bin << 2 | lvl;
+                out_n[z] += (uint32_t)__popc(bal);
             }
-            if (n > slot) {
-                if (lane == 0) atomicOr(err, kErrListOverflow);
-                n = slot;
-            }
-            if (lane == 0) list_len[(size_t)(z - 1) * db.num_pep + p] = (uint16_t)min(n, 65535);
-            my_lists += 1u;
-            my_entries += (uint32_t)n;
-            __syncwarp();
         }
+#pragma unroll
+        for (int z = 0; z < kLevels; ++z)
+            if ((need >> z) & 1u) {
+                if (lane == 0) list_len[(size_t)z * db.num_pep + p] = (uint16_t)out_n[z];
+                my_lists += 1u;
+                my_entries += out_n[z];
+            }
+        __syncwarp();
     }
     if (stats) {
         if (lane == 0) {
@@ -805,7 +739,7 @@ int hfx_lists_generate(const DevDB &db, const int32_t *cover, int64_t npep1, int
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const WorkLists wl{work, db.num_pep};
     cudaMemsetAsync(work, 0, 16, st);
-    k_list_work<<<(db.num_pep + 255) / 256, 256, 0, st>>>(db, cover, npep1, list_len, wl);
+    k_list_work<false><<<(db.num_pep + 255) / 256, 256, 0, st>>>(db, cover, npep1, list_len, wl, nullptr);
     auto run = [&](auto f, int most) {
         cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         int per = 0;
@@ -932,19 +866,26 @@ int hfx_lists_score(const void *lists, int long_rows, const uint32_t *lstart, ui
 
 int hfx_lists_generate_long(const DevDB &db, const int32_t *cover, int64_t npep1, int32_t nbins,
                             const uint32_t *lstart, uint64_t total10, uint32_t *lists, uint16_t *list_len,
-                            int fastdiv, float ion_bw, unsigned long long *stats, uint32_t *err,
+                            uint32_t *work, int fastdiv, float ion_bw, unsigned long long *stats, uint32_t *err,
                             cudaStream_t st) {
-    const int nw = 8;
-    const size_t smem = (size_t)nw * kLongKeys * 4;
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    auto f = fastdiv ? k_gen_lists_long<true> : k_gen_lists_long<false>;
-    cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    int per = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, f, nw * 32, smem);
-    f<<<sms * (per > 0 ? per : 1), nw * 32, smem, st>>>(db, cover, npep1, nbins, lstart, total10, lists, list_len,
-                                                        ion_bw, stats, err);
+    const WorkLists wl{work, db.num_pep};
+    cudaMemsetAsync(work, 0, 16, st);
+    k_list_work<true><<<(db.num_pep + 255) / 256, 256, 0, st>>>(db, cover, npep1, list_len, wl, err);
+    const float width = ion_bw > 0.0f ? ion_bw : kBinMono;
+    auto run = [&](auto f, int cls, int nw) {
+        const size_t smem = (size_t)nw * long_bytes(cls);
+        cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        int per = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, f, nw * 32, smem);
+        f<<<sms * std::max(1, per), nw * 32, smem, st>>>(db, nbins, lstart, total10, lists, list_len, width, wl,
+                                                         stats);
+    };
+    run(fastdiv ? k_gen_lists_long<true, 1> : k_gen_lists_long<false, 1>, 1, 8);
+    run(fastdiv ? k_gen_lists_long<true, 2> : k_gen_lists_long<false, 2>, 2, 4);
+    run(fastdiv ? k_gen_lists_long<true, 0> : k_gen_lists_long<false, 0>, 0, 2);
     return (int)cudaGetLastError();
 }
 

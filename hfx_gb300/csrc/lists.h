@@ -38,7 +38,7 @@ int hfx_lists_group_fits(int32_t G, int long_rows, int64_t stride, int elem_byte
 // and FP32 rescoring of kept unmodified candidates from those lists.
 int hfx_lists_generate_long(const hfx::DevDB &db, const int32_t *cover, int64_t npep1, int32_t nbins,
                             const uint32_t *lstart, uint64_t total10, uint32_t *lists, uint16_t *list_len,
-                            int fastdiv, float ion_bw, unsigned long long *stats, uint32_t *err,
+                            uint32_t *work, int fastdiv, float ion_bw, unsigned long long *stats, uint32_t *err,
                             cudaStream_t st);
 // FP32 rescoring of kept unmodified candidates from the step's lists (32-bit
 // entries for long rows, else 16-bit) and the FP32 rows.

@@ -82,6 +82,17 @@ __device__ __forceinline__ uint4 lds_u128(uint32_t a) {
 __device__ __forceinline__ void sts_u16(uint32_t a, uint32_t v) {
     asm volatile("st.shared.u16 [%0], %1;" ::"r"(a), "h"((uint16_t)v) : "memory");
 }
+__device__ __forceinline__ void sts_u32(uint32_t a, uint32_t v) {
+    asm volatile("st.shared.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+__device__ __forceinline__ void red_add(uint32_t a, uint32_t v) {
+    asm volatile("red.shared.add.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+__device__ __forceinline__ uint32_t atom_add(uint32_t a, uint32_t v) {
+    uint32_t o;
+    asm volatile("atom.shared.add.u32 %0, [%1], %2;" : "=r"(o) : "r"(a), "r"(v) : "memory");
+    return o;
+}
 __device__ __forceinline__ void sts_u128(uint32_t a, uint4 v) {
     asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w)
                  : "memory");
@@ -153,7 +164,7 @@ struct ItemBits {
 // Correctly rounded a / d from y = RN(1 / d): q = RN(a y) is within an ulp, the
 // remainder a - q d is exact in one FMA, and q + remainder y rounds to the
 // quotient (Markstein, IBM J. Res. Dev. 34, 1990).  Equal to the IEEE division
-// for d = 1.0005079 and d = 3 and every float in [2^-12, 2^22], which is where
+// for d = 1.0005079, 0.02 and 3 and every float in [2^-12, 2^22], which is where
 // the ions lie (tests/test_lists_math.py; an infinite a would give a NaN, so
 // masses from 2^22 on take the other path).  Three instructions and no branch;
 // the division's own slow path is a call, which costs a kernel that keeps a

@@ -13,12 +13,12 @@ pytestmark = pytest.mark.gpu
 LENGTHS = [1, 2, 6, 16, 17, 31, 32, 33, 34, 50, 63, 64, 65, 66, 96, 97, 130]
 
 
-def _database(seed):
+def _database(seed, longest=130):
     rng = np.random.default_rng(seed)
     letters = np.frombuffer(b"ACDEFGHIKLMNPQRSTVWYUBZX", np.uint8)
     seq = letters[rng.integers(0, len(letters), size=4000)].astype(np.uint8)
     tc, tn = [], []
-    for k, n in enumerate(LENGTHS * 2):
+    for k, n in enumerate([n for n in LENGTHS * 2 if n <= longest]):
         a = int(rng.integers(0, 4000 - 140))
         tc.append(a)
         tn.append(a + n)
@@ -59,6 +59,30 @@ def test_lists_at_their_edges(gpulib, oracle, top_mz, precision):
                        *(np.concatenate([getattr(p, f) for p in parts]) for f in ("pcr", "z", "tol")))
     res = eng.search(sp, hfx_gb300.default_params(top_n=32, batch_mode=1, precision=precision, rescore_k=64))
     sc, _, key, pep, nc = oracle.search(oracle.pack_ions(seq), mt, rs, tcs, tns, idx, sp, topn=32)
+    assert np.array_equal(res.ncand, nc)
+    assert np.array_equal(res.key, key)
+    assert np.array_equal(res.score.view(np.uint32), sc.view(np.uint32))
+    eng.close()
+
+
+@pytest.mark.parametrize("custom", [0, 1])
+@pytest.mark.parametrize("width", [0.02, 0.0137])
+def test_long_row_lists_at_their_edges(gpulib, oracle, width, custom):
+    """Rows beyond 8,192 bins: peptides around 1,024 and 2,048 keys (10 keys a
+    prefix and charge) and up to 4,000, both ion widths."""
+    import hfx_gb300
+    seq, r, tc, tn, mt = _database(5, longest=100)
+    eng = hfx_gb300.Engine(0)
+    eng.upload_db(seq, r, tc, tn, mt)
+    rs, tcs, tns, idx, _ = eng.db_export()
+    parts = [_spectra(10 * c + 1, c, 1200.0) for c in (1, 2, 3, 4, 5)]
+    off = np.concatenate([[0], np.cumsum(np.concatenate([np.diff(p.off) for p in parts]))]).astype(np.int64)
+    sp = synth.Spectra(*(np.concatenate([getattr(p, f) for p in parts]) for f in ("mz", "it")), off,
+                       *(np.concatenate([getattr(p, f) for p in parts]) for f in ("pcr", "z", "tol")))
+    p = hfx_gb300.default_params(top_n=32, batch_mode=1, bin_width=width, custom_bin_width=1, ion_bins_custom=custom)
+    res = eng.search(sp, p)
+    sc, _, key, pep, nc = oracle.search(oracle.pack_ions(seq), mt, rs, tcs, tns, idx, sp, topn=32, bw=width,
+                                        custom_bw=True, ion_bw=width if custom else 0.0)
     assert np.array_equal(res.ncand, nc)
     assert np.array_equal(res.key, key)
     assert np.array_equal(res.score.view(np.uint32), sc.view(np.uint32))

@@ -12,7 +12,7 @@ def _rn(x: Fraction) -> np.float32:
     return np.float32(float(x))
 
 
-@pytest.mark.parametrize("d", [1.0005079, 1.0, 2.0, 3.0, 4.0])
+@pytest.mark.parametrize("d", [1.0005079, 0.02, 0.0137, 1.0, 2.0, 3.0, 4.0])
 def test_corrected_quotient_is_the_ieee_quotient(d):
     d = np.float32(d)
     y = np.float32(1.0) / d
