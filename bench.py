@@ -46,7 +46,7 @@ sys.path.insert(0, ROOT)
 
 METRIC = "peptide-spectrum XCorrs/s"
 UNIT = "PSM/s"
-KERNELS = {0: "k_score_spectrum", 1: "k_score_lists", 2: "k_score_batched"}
+KERNELS = {0: "k_score_spectra", 1: "k_score_lists", 2: "k_score_batched"}
 
 # DRAM bytes (read + write) per launch, from ncu captures (summaries under
 # profiles/), keyed by (kernel, workload, precision, spectra).  Each figure
@@ -91,7 +91,7 @@ def _args():
     ap.add_argument("--spectra", type=int, default=0, help="override the number of spectra")
     ap.add_argument("--precision", type=int, default=1, help="0 fp32, 1 bf16+rescore, 2 fp16+rescore")
     ap.add_argument("--batch-mode", type=int, default=1,
-                    help="0 per-spectrum launches, 1 batched over ion lists, 2 batched fused")
+                    help="0 per-spectrum blocks, 1 batched over ion lists, 2 batched fused")
     ap.add_argument("--cpu-sample", type=int, default=-1,
                     help="spectra in the CPU baseline sample (-1: whole 'full' workload, 300 otherwise)")
     ap.add_argument("--agree-sample", type=int, default=-1,
@@ -526,10 +526,10 @@ def main():
         eng.search(Pinned(), p)
         e2e_tot += time.perf_counter() - t1
     e2e_value = psm_all / (e2e_tot / a.e2e_steps)
-    # the plain FP32 path (one launch per spectrum) on the same spectra
+    # the plain FP32 path (every spectrum by its own blocks) on the same spectra
     plain = None
     if not a.no_plain and not has_mods:
-        # the plain FP32 path: one launch per spectrum (rows beyond 8192 bins
+        # the plain FP32 path: every spectrum by its own blocks (rows beyond 8192 bins
         # always take the batched list path, there in FP32)
         p0 = hfx_gb300.default_params(top_n=tn_, precision=0, batch_mode=0, **_pkw(cfg))
         n_pl = min(ns, plain_n)
@@ -665,7 +665,7 @@ def main():
                    "precision": ["fp32", "bf16 store, fp32 accumulate, fp32 rescore",
                                  "fp16 store, fp32 accumulate, fp32 rescore"][prec]
                    + (f" of the top {rk}" if prec else ""),
-                   "batch_mode": ["per-spectrum launches", "batched over ion lists", "batched fused"][mode],
+                   "batch_mode": ["per-spectrum blocks", "batched over ion lists", "batched fused"][mode],
                    "launch": "one CUDA-graph replay per step" if graph else "eager launches",
                    "autotuned": tuned,
                    "l2": "flushed between timed steps (512 MB write)",

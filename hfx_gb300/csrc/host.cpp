@@ -479,20 +479,14 @@ int32_t search_plain_per_spectrum(hfx_ctx *ctx, const hfx_search_params *p, cons
     if (e) return cuda_fail(ctx, e, "alloc part_off");
     HFX_CUDA(cudaMemcpyAsync(d_off, part_off.data(), 8ull * (b.nspec + 1), cudaMemcpyHostToDevice, ctx->stream),
              "H2D part_off");
-    const DevDB db = ctx->devdb();
-    int64_t nl = 0, psm = 0;
+    int64_t psm = 0;
+    for (int32_t s = 0; s < b.nspec; ++s)
+        if (nblk[s] > 0) psm += he[s] - hb[s];
     ctx->stage_begin(HFX_STAGE_SCORE);
-    for (int32_t s = 0; s < b.nspec; ++s) {
-        if (nblk[s] == 0) continue;
-        ++nl;
-        psm += he[s] - hb[s];
-        const int32_t ch = hm[s].charges_plain;
-        rc = hfx_launch_score_spectrum(db, rows + (size_t)s * stride, hm[s].len, ch, hb[s], he[s], K, nblk[s],
-                                       p->fastdiv, ps + part_off[s] * K, pk + part_off[s] * K,
-                                       ctx->d_err.as<uint32_t>(), ctx->stream);
-        if (rc) return cuda_fail(ctx, (cudaError_t)rc, "k_score_spectrum");
-    }
-    ctx->stage_end(HFX_STAGE_SCORE, nl, psm);
+    rc = hfx_launch_score_spectra(ctx->devdb(), rows, stride, meta, wb, we, d_off, b.nspec, part_off[b.nspec], K,
+                                  p->fastdiv, ps, pk, ctx->stream);
+    if (rc) return cuda_fail(ctx, (cudaError_t)rc, "k_score_spectra");
+    ctx->stage_end(HFX_STAGE_SCORE, part_off[b.nspec] > 0 ? 1 : 0, psm);
     ctx->stage_begin(HFX_STAGE_TOPN);
     rc = hfx_launch_merge_parts(ps, pk, d_off, b.nspec, K, p->top_n, ctx->d_idx.as<uint32_t>(), out_s, out_k,
                                 out_pep, ctx->stream);
