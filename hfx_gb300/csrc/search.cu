@@ -119,17 +119,24 @@ __global__ void __launch_bounds__(256) k_score_spectra(DevDB db, const float *__
     }
 }
 
-// Merge per-spectrum partial lists into the final top-N.
-__global__ void k_merge_parts(const float *__restrict__ part_s, const uint64_t *__restrict__ part_k,
+// Merge per-spectrum partial lists into the final top-N, a block each.
+constexpr int kPartWarps = 4;
+__global__ void __launch_bounds__(32 * kPartWarps) k_merge_parts(const float *__restrict__ part_s, const uint64_t *__restrict__ part_k,
                               const int64_t *__restrict__ part_off, int32_t nspec, int32_t K, int32_t topn,
                               const uint32_t *__restrict__ idx_sorted, float *__restrict__ out_s,
                               uint64_t *__restrict__ out_k, uint32_t *__restrict__ out_pep) {
-    const int lane = threadIdx.x & 31;
-    const int32_t s = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (s >= nspec) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int32_t s = blockIdx.x;
+    __shared__ float sm_s[kPartWarps][32];
+    __shared__ uint64_t sm_k[kPartWarps][32];
     WarpList32 tk;
     tk.init();
-    for (int64_t b = part_off[s]; b < part_off[s + 1]; ++b) tk.merge_list(part_s + b * K, part_k + b * K, K);
+    for (int64_t b = part_off[s] + warp; b < part_off[s + 1]; b += kPartWarps)
+        tk.merge_list(part_s + b * K, part_k + b * K, K);
+    if (warp > 0) tk.store(sm_s[warp], sm_k[warp], 32);
+    __syncthreads();
+    if (warp > 0) return;
+    for (int w = 1; w < kPartWarps; ++w) tk.merge_list(sm_s[w], sm_k[w], 32);
     if (lane < topn) {
         out_s[(size_t)s * topn + lane] = tk.s;
         out_k[(size_t)s * topn + lane] = tk.k;
@@ -233,7 +240,7 @@ int hfx_launch_merge_parts(const float *part_s, const uint64_t *part_k, const in
                            int32_t K, int32_t topn, const uint32_t *idx_sorted, float *out_s, uint64_t *out_k,
                            uint32_t *out_pep, cudaStream_t st) {
     if (nspec <= 0) return 0;
-    k_merge_parts<<<(nspec + 3) / 4, 128, 0, st>>>(part_s, part_k, part_off, nspec, K, topn, idx_sorted, out_s,
+    k_merge_parts<<<nspec, 32 * kPartWarps, 0, st>>>(part_s, part_k, part_off, nspec, K, topn, idx_sorted, out_s,
                                                    out_k, out_pep);
     return (int)cudaGetLastError();
 }
