@@ -23,6 +23,7 @@
 #include "batched_common.cuh"
 #include "mods_device.cuh"
 #include "scan.cuh"
+#include "dense.h"
 #include <type_traits>
 
 namespace hfx {
@@ -114,8 +115,8 @@ __global__ void k_bucket_scatter(const SpecMeta *__restrict__ meta, int32_t nspe
 // With few_groups (no work-item size asked for) a group's window is cut so
 // that about this many items come of all groups together, four per resident
 // CTA of the list scorer: one spectrum's 3,400 candidates in one item kept one
-// SM busy for 0.22 ms.  From about 1,200 groups (76 of open windows) on the rule
-// changes nothing.
+// SM busy for 0.22 ms.  Groups of narrow and of wide windows count apart; from
+// about 1,200 groups (76 of open windows) on the rule changes nothing.
 constexpr uint32_t kFewItems = 1216;
 
 // One thread per group: members, union window, chunk count.
@@ -159,6 +160,7 @@ __global__ void k_groups(const uint32_t *__restrict__ bucket_end, const uint32_t
     gi.maxlen = 0;
     gi.charges = 0;
     gi.charges_mod = 0;
+    gi.block = -1;
     for (uint32_t j = 0; j < cnt; ++j) {
         const int32_t s = perm[pos0 + j];
         group_of[s] = g;
@@ -184,7 +186,9 @@ __global__ void k_groups(const uint32_t *__restrict__ bucket_end, const uint32_t
                                                     : chunk;
     gi.chunk = group_chunk(gi.hi - gi.lo, cg);
     if (few_groups) {
-        const uint64_t share = ((uint64_t)(gi.hi - gi.lo) * ng + kFewItems - 1) / kFewItems;
+        uint32_t alike = 0;  // groups whose windows are as wide (narrow classes are even, wide ones odd)
+        for (int k = c & 1; k < kClasses; k += 2) alike += grp_start[k + 1] - grp_start[k];
+        const uint64_t share = ((uint64_t)(gi.hi - gi.lo) * alike + kFewItems - 1) / kFewItems;
         gi.chunk = (uint32_t)min((uint64_t)gi.chunk, max(share, (uint64_t)64));
     }
     groups[g] = gi;
@@ -294,26 +298,78 @@ k_score_batched(DevDB db, const T *__restrict__ tiles, int64_t stride, const uin
     }
 }
 
-// Per spectrum: merge its slot of every item of its group.
-// R = 1: up to 32 kept per spectrum (WarpTopK), R = 2: up to 64 (WarpTopK64).
+// Per spectrum: merge its slot of every item of its group that its window
+// reaches, a block of kMergeWarps warps each (one warp over all items of the
+// group took 38 us for one spectrum's 53 items, and the windows of a few
+// spectra far apart in mass have hundreds).
+// R = 1: up to 32 kept per spectrum, R = 2: up to 64.
+constexpr int kMergeWarps = 4;
 template <int R>
-__global__ void k_merge_items(const float *__restrict__ part_s, const uint64_t *__restrict__ part_k,
+__global__ void __launch_bounds__(32 * kMergeWarps) k_merge_items(const float *__restrict__ part_s, const uint64_t *__restrict__ part_k,
                               const uint32_t *__restrict__ item_off, const int32_t *__restrict__ group_of,
-                              const int32_t *__restrict__ slot_of, const SpecMeta *__restrict__ meta, int32_t nspec,
-                              int32_t G, int32_t K, int32_t kout, float *__restrict__ out_s,
-                              uint64_t *__restrict__ out_k) {
-    const int lane = threadIdx.x & 31;
-    const int32_t s = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (s >= nspec) return;
+                              const int32_t *__restrict__ slot_of, const SpecMeta *__restrict__ meta,
+                              const uint32_t *__restrict__ wb, const uint32_t *__restrict__ we, int32_t G, int32_t K,
+                              int32_t kout, float *__restrict__ out_s,
+                              uint64_t *__restrict__ out_k, const GroupInfo *__restrict__ groups,
+                              const unsigned long long *__restrict__ dense,
+                              const unsigned long long *__restrict__ dense_left,
+                              const DenseBlock *__restrict__ blocks, const uint32_t *__restrict__ dense_off) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int32_t s = blockIdx.x;
+    __shared__ float sm_s[kMergeWarps][32 * R];
+    __shared__ uint64_t sm_k[kMergeWarps][32 * R];
     typename std::conditional<R == 1, WarpList32, WarpList64>::type tk;
     tk.init();
     if (meta[s].status == 0) {
         const int32_t g = group_of[s], j = slot_of[s];
-        for (uint32_t it = item_off[g]; it < item_off[g + 1]; ++it) {
-            const size_t o = ((size_t)it * G + j) * K;
-            tk.merge_list(part_s + o, part_k + o, K);
+        // the items that overlap the spectrum's own window, a warp each in turn
+        const GroupInfo gi = groups[g];
+        const uint32_t i0 = item_off[g], i1 = item_off[g + 1];
+        if (we[s] > wb[s] && i1 > i0) {
+            const uint32_t last = min(i1 - 1u, i0 + (we[s] - 1u - gi.lo) / gi.chunk);
+            for (uint32_t it = i0 + (wb[s] - gi.lo) / gi.chunk + (uint32_t)warp; it <= last; it += nw) {
+                const size_t o = ((size_t)it * G + j) * K;
+                tk.merge_list(part_s + o, part_k + o, K);
+            }
+        }
+        // a block scored on the tensor cores: the spectrum's list and what the
+        // block's items had left over (unsorted, up to 16 each)
+        if constexpr (R == 1) {
+            const int32_t b = dense ? gi.block : -1;
+            if (b >= 0) {
+                auto take = [&](unsigned long long x) {
+                    const uint32_t o = (uint32_t)(x >> 32);
+                    tk.merge(x ? __uint_as_float((o & 0x80000000u) ? (o & 0x7FFFFFFFu) : ~o) : -INFINITY,
+                             x ? (uint64_t)(uint32_t)~(uint32_t)x : ~0ull);
+                };
+                if (warp == 0) take(dense[(size_t)s * 32 + lane]);
+                const uint32_t m = gi.pos0 + (uint32_t)j - blocks[b].pos0;
+                for (uint32_t it = dense_off[b] + 2u * (uint32_t)warp; it < dense_off[b + 1]; it += 2u * nw) {
+                    // two items at a time, 32 entries sorted best first
+                    const uint32_t mine = it + (uint32_t)(lane >> 4);
+                    unsigned long long x =
+                        mine < dense_off[b + 1]
+                            ? dense_left[((size_t)mine * kDenseSpectra + m) * kDenseQueue + (lane & 15)]
+                            : 0ull;
+                    if (!__any_sync(kFullMask, x != 0ull)) continue;
+#pragma unroll
+                    for (int w = 2; w <= 32; w <<= 1)
+#pragma unroll
+                        for (int d = w >> 1; d > 0; d >>= 1) {
+                            const unsigned long long y = __shfl_xor_sync(kFullMask, x, d);
+                            const bool high = ((lane & d) == 0) == ((lane & w) == 0);
+                            x = high ? max(x, y) : min(x, y);
+                        }
+                    take(x);
+                }
+            }
         }
     }
+    // the warps' lists into the first
+    if (warp > 0) tk.store(sm_s[warp], sm_k[warp], 32 * R);
+    __syncthreads();
+    if (warp > 0) return;
+    for (int w = 1; w < nw; ++w) tk.merge_list(sm_s[w], sm_k[w], 32 * R);
     tk.store(out_s + (size_t)s * kout, out_k + (size_t)s * kout, kout);
 }
 
@@ -441,7 +497,7 @@ size_t hfx_batched_smem(int64_t stride, int elem_bytes, int G, int nw, int K) {
 }
 
 int hfx_batched_plan(const SpecMeta *meta, int32_t nspec, const uint32_t *wb, const uint32_t *we, int32_t G,
-                     int32_t chunk, int few_groups, const BatchedWs &ws, cudaStream_t st) {
+                     int32_t chunk, int few_groups, const BatchedWs &ws, const DenseWs *dw, cudaStream_t st) {
     const int nbk = kClasses * kMassBuckets;
     cudaMemsetAsync(ws.hist, 0, sizeof(uint32_t) * (nbk + 1), st);
     cudaMemsetAsync(ws.item_off, 0, sizeof(uint32_t) * (nspec + 1), st);
@@ -452,6 +508,11 @@ int hfx_batched_plan(const SpecMeta *meta, int32_t nspec, const uint32_t *wb, co
     k_groups<<<(max_groups + 255) / 256, 256, 0, st>>>(ws.hist, ws.n_sorted, ws.perm, wb, we, meta, G, chunk,
                                                        few_groups, max_groups, ws.groups, ws.item_off, ws.group_of, ws.slot_of,
                                                        ws.ngroups);
+    if (dw) {
+        const int rc = hfx_dense_plan(meta, nspec, wb, we, G, ws.hist, ws, ws.item_off, *dw, st);
+        if (rc) return rc;
+        k_scan_u32<<<1, 1024, 0, st>>>(dw->item_off, dw->cap_blocks + 1, dw->total_items);
+    }
     k_scan_u32<<<1, 1024, 0, st>>>(ws.item_off, max_groups + 1, ws.total_items);
     return (int)cudaGetLastError();
 }
@@ -556,15 +617,20 @@ int hfx_clamp_items(uint32_t *off, int64_t n1, uint32_t cap, uint32_t *err, cuda
 }
 
 int hfx_batched_merge(const float *part_s, const uint64_t *part_k, const BatchedWs &ws, const SpecMeta *meta,
-                      int32_t nspec, int32_t G, int32_t K, int32_t kout, float *out_s, uint64_t *out_k,
-                      cudaStream_t st) {
+                      const uint32_t *wb, const uint32_t *we, int32_t nspec, int32_t G, int32_t K, int32_t kout,
+                      float *out_s, uint64_t *out_k,
+                      const DenseWs *dw, cudaStream_t st) {
     if (kout > kMaxKept || K > kMaxKept) return (int)cudaErrorInvalidValue;
     if (kout > 32 || K > 32)
-        k_merge_items<2><<<(nspec + 3) / 4, 128, 0, st>>>(part_s, part_k, ws.item_off, ws.group_of, ws.slot_of, meta,
-                                                          nspec, G, K, kout, out_s, out_k);
+        k_merge_items<2><<<nspec, 32 * kMergeWarps, 0, st>>>(part_s, part_k, ws.item_off, ws.group_of, ws.slot_of, meta,
+                                                          wb, we, G, K, kout, out_s, out_k, ws.groups,
+                                                          dw ? dw->best : nullptr, dw ? dw->left : nullptr,
+                                                          dw ? dw->blocks : nullptr, dw ? dw->item_off : nullptr);
     else
-        k_merge_items<1><<<(nspec + 3) / 4, 128, 0, st>>>(part_s, part_k, ws.item_off, ws.group_of, ws.slot_of, meta,
-                                                          nspec, G, K, kout, out_s, out_k);
+        k_merge_items<1><<<nspec, 32 * kMergeWarps, 0, st>>>(part_s, part_k, ws.item_off, ws.group_of, ws.slot_of, meta,
+                                                          wb, we, G, K, kout, out_s, out_k, ws.groups,
+                                                          dw ? dw->best : nullptr, dw ? dw->left : nullptr,
+                                                          dw ? dw->blocks : nullptr, dw ? dw->item_off : nullptr);
     return (int)cudaGetLastError();
 }
 

@@ -10,6 +10,7 @@ struct GroupInfo {
     int32_t charges;       // ion charges shared by the members (unmodified)
     int32_t charges_mod;   // ion charges of the members' modified candidates
     uint32_t chunk;        // candidates per work item of this group
+    int32_t block;         // its block when that is scored on the tensor cores (dense.h), else -1
 };
 
 struct BatchedWs {
@@ -26,11 +27,12 @@ struct BatchedWs {
 };
 
 constexpr int kBucketCount = 12 * 8192;
+struct DenseWs;
 }  // namespace hfx
 
 size_t hfx_batched_smem(int64_t stride, int elem_bytes, int G, int nw, int K);
 int hfx_batched_plan(const hfx::SpecMeta *meta, int32_t nspec, const uint32_t *wb, const uint32_t *we, int32_t G,
-                     int32_t chunk, int few_groups, const hfx::BatchedWs &ws, cudaStream_t st);
+                     int32_t chunk, int few_groups, const hfx::BatchedWs &ws, const hfx::DenseWs *dw, cudaStream_t st);
 // Runs the persistent scorer over the group tiles packed by hfx_pack_tiles
 // (tiles: ngroups * stride * G elements); nw = warps per CTA (0 = as many as shared memory holds,
 // at most 16), grid = CTAs (0 = one wave).
@@ -43,8 +45,9 @@ int hfx_clamp_items(uint32_t *off, int64_t n1, uint32_t cap, uint32_t *err, cuda
 // it and sets kErrBounds in the error word.
 int hfx_clamp_groups(uint32_t *ngroups, uint32_t cap, uint32_t *err, cudaStream_t st);
 int hfx_batched_merge(const float *part_s, const uint64_t *part_k, const hfx::BatchedWs &ws,
-                      const hfx::SpecMeta *meta, int32_t nspec, int32_t G, int32_t K, int32_t kout, float *out_s,
-                      uint64_t *out_k, cudaStream_t st);
+                      const hfx::SpecMeta *meta, const uint32_t *wb, const uint32_t *we, int32_t nspec, int32_t G,
+                      int32_t K, int32_t kout, float *out_s, uint64_t *out_k, const hfx::DenseWs *dw,
+                      cudaStream_t st);
 // FP32 rescoring of the kept low-precision matches (unmodified and modified
 // keys) and the final top-N.
 int hfx_rescore(const hfx::DevDB &db, const hfx::DevMods &mods, const float *rows32, int64_t stride,

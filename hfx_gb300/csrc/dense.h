@@ -1,0 +1,58 @@
+// Tensor-core scoring of wide windows (dense.cu): declarations.
+#pragma once
+#include "hfx_internal.h"
+#include "batched.h"
+
+namespace hfx {
+
+constexpr int kDenseSpectra = 128;  // spectra per block: the rows of one MMA
+constexpr int kDenseQueue = 16;     // queued candidates per spectrum
+
+// A run of up to 128 spectra of one class, neighbours in the planned order.
+struct DenseBlock {
+    uint32_t pos0, count;  // members: perm[pos0 .. pos0 + count)
+    uint32_t lo, hi;       // union of their candidate windows
+    int32_t maxlen, charges;
+    uint32_t chunk;        // candidates per work item
+    uint32_t tile;         // index of its operand tile
+};
+
+struct DenseWs {
+    DenseBlock *blocks;    // [cap_blocks]
+    uint32_t *item_off;    // [cap_blocks + 1]: first work item of each block (blocks that are not dense have none)
+    uint32_t *tile_block;  // [cap_blocks]: block of each operand tile
+    uint32_t *n_tiles;     // [1]
+    uint32_t *total_items; // [1]
+    uint32_t *counter;     // [1] work-stealing cursor
+    unsigned long long *best;  // [nspec][32] each spectrum's best candidates so far, descending: score order << 32 | ~position
+    unsigned long long *left;  // [items][128][kDenseQueue] candidates an item did not merge into it (0: none)
+    uint32_t *lock;        // [nspec] of that list
+    uint32_t *thr;         // [nspec] its K-th score (ordered bits, 0 = none yet)
+    int32_t cap_blocks;
+};
+
+// Blocks of nspec spectra (every class may end in a partial one).
+constexpr int32_t dense_blocks(int32_t nspec) { return nspec / kDenseSpectra + 13; }
+// 128-bin chunks of a row, and the bytes of one operand tile.
+constexpr int64_t dense_chunks(int64_t stride) { return (stride + 127) / 128; }
+constexpr size_t dense_tile_bytes(int64_t stride, int pieces) {
+    return (size_t)dense_chunks(stride) * pieces * kDenseSpectra * 128;
+}
+
+}  // namespace hfx
+
+// 8-bit pieces a row value is split into for a row precision (0 FP32, 1 BF16, 2 FP16).
+int hfx_dense_pieces(int elem_kind);
+// Marks the blocks whose windows overlap enough (their groups get no work
+// items of their own) and cuts them into items; between k_groups and the scan
+// of the groups' items.
+int hfx_dense_plan(const hfx::SpecMeta *meta, int32_t nspec, const uint32_t *wb, const uint32_t *we, int32_t G,
+                   const uint32_t *bucket_end, const hfx::BatchedWs &ws, uint32_t *nchunks, const hfx::DenseWs &dw,
+                   cudaStream_t st);
+int hfx_dense_pack(const float *rows, int64_t stride, const hfx::BatchedWs &ws, const hfx::DenseWs &dw,
+                   uint32_t cap_tiles, int pieces, uint8_t *tiles, uint32_t *err, cudaStream_t st);
+int hfx_dense_score(const uint16_t *lists, uint64_t list_total, const uint32_t *lstart, uint64_t total10,
+                    const uint16_t *list_len, uint32_t num_pep, const uint8_t *tiles, uint32_t cap_tiles,
+                    int64_t stride, int pieces, const uint32_t *wb, const uint32_t *we, int32_t nspec,
+                    const hfx::BatchedWs &ws, const hfx::DenseWs &dw, int32_t K, unsigned long long *stats, uint32_t *err,
+                    cudaStream_t st);

@@ -27,6 +27,7 @@ struct SpecMeta {
     int32_t npk, len, status;
     float cutoff, mass, eps, lo, hi;
     int32_t charges_plain, charges_mod;
+    int32_t nonfinite;  // a kept peak's intensity is infinite (its row holds NaN)
 };
 
 // Search database on the device, in residual-mass order.
@@ -64,6 +65,6 @@ int hfx_launch_layout(const float *mz, const int64_t *off, const float *pcr, con
                       const float *tol, int32_t nspec, const hfx::LayoutParams &lp,
                       hfx::SpecMeta *meta, uint32_t *max_len, uint32_t *err, cudaStream_t st);
 int hfx_launch_preprocess(const float *mz, const float *it, const int64_t *off, const float *pcr,
-                          const hfx::LayoutParams &lp, const hfx::SpecMeta *meta, int32_t nspec,
+                          const hfx::LayoutParams &lp, hfx::SpecMeta *meta, int32_t nspec,
                           int64_t stride, float *out32, __nv_bfloat16 *outbf, __half *outh, uint32_t *err,
                           cudaStream_t st);

@@ -14,6 +14,7 @@
 #include "evalues.h"
 #include "ions.h"
 #include "iso_lists.h"
+#include "dense.h"
 
 int hfx_digest_launch(const uint8_t *d_seq, const uint32_t *d_seg, int32_t nprot, uint32_t nres, const float *mt26,
                       int32_t rule_mask, int32_t missed, float min_mass, float max_mass, int32_t proline,
@@ -147,6 +148,7 @@ struct hfx_ctx {
     int64_t rows_stride = 0;
     int32_t rows_nspec = 0;
     uint32_t last_items = 0, last_mitems = 0;
+    uint32_t last_tiles = 0, cap_tiles = 0, last_ditems = 0, cap_ditems = 0;  // dense blocks: operand tiles, items
     bool graph_valid = false;
     cudaGraphExec_t graph_exec = nullptr;
     cudaStream_t graph_stream = nullptr;  // captures and replays run here (never the legacy stream)
@@ -602,7 +604,7 @@ int32_t search_batched(hfx_ctx *ctx, const hfx_search_params *p, const Batch &b,
     // candidates kept for FP32 rescoring: up to 64 when unmodified candidates
     // alone are list-scored in groups of up to 8, else up to 32
     const bool lists_only = (p->batch_mode == 1 || long_rows) && !(p->search_mods != 0 && ctx->num_mod > 0);
-    const int32_t K = elem_kind == 0 ? p->top_n
+    int32_t K = elem_kind == 0 ? p->top_n
                                      : std::max(p->top_n, std::min(p->rescore_k > 0 ? p->rescore_k : 32,
                                                                    lists_only ? kMaxKept : kMaxTopK));
     if (K > 32 && G == 16) G = 8;
@@ -628,6 +630,25 @@ int32_t search_batched(hfx_ctx *ctx, const hfx_search_params *p, const Batch &b,
     if (e) return cuda_fail(ctx, e, "alloc");
     uint32_t *scal = ctx->buf<uint32_t>("b_scal", 8, e);
     if (e) return cuda_fail(ctx, e, "alloc");
+    // wide windows on the tensor cores: unmodified candidates, lists, up to 32
+    // kept, and without a score sink; an FP32 search keeps 32 then and rescores
+    // them, so it has to ask for few enough of them
+    const bool dense_on = lists_only && !long_rows && K <= 32 && p->search_plain != 0 &&
+                          (elem_kind != 0 || (p->top_n <= 16 && !ctx->ev_single));
+    DenseWs dw{};
+    if (dense_on) {
+        dw.cap_blocks = dense_blocks(ns);
+        dw.blocks = ctx->buf<DenseBlock>("d_blocks", dw.cap_blocks, e);
+        dw.item_off = e ? nullptr : ctx->buf<uint32_t>("d_itemoff", (size_t)dw.cap_blocks + 1, e);
+        dw.tile_block = e ? nullptr : ctx->buf<uint32_t>("d_tileblock", dw.cap_blocks, e);
+        dw.thr = e ? nullptr : ctx->buf<uint32_t>("d_thr", ns, e);
+        dw.lock = e ? nullptr : ctx->buf<uint32_t>("d_lock", ns, e);
+        dw.best = e ? nullptr : ctx->buf<unsigned long long>("d_best", 32ull * ns, e);
+        if (e) return cuda_fail(ctx, e, "alloc");
+        dw.n_tiles = scal + 4;
+        dw.total_items = scal + 5;
+        dw.counter = scal + 6;
+    }
     ws.n_sorted = scal;
     ws.ngroups = scal + 1;
     ws.total_items = scal + 2;
@@ -645,10 +666,11 @@ int32_t search_batched(hfx_ctx *ctx, const hfx_search_params *p, const Batch &b,
     ctx->stage_begin(HFX_STAGE_WINDOWS);
     int rc = hfx_launch_windows(ctx->d_r.as<float>(), (uint32_t)ctx->num_pep, meta, ns, wb, we, ctx->stream);
     if (rc) return cuda_fail(ctx, (cudaError_t)rc, "k_windows");
-    rc = hfx_batched_plan(meta, ns, wb, we, G, chunk, p->chunk > 0 ? 0 : 1, ws, ctx->stream);
+    rc = hfx_batched_plan(meta, ns, wb, we, G, chunk, p->chunk > 0 ? 0 : 1, ws, dense_on ? &dw : nullptr,
+                          ctx->stream);
     if (rc) return cuda_fail(ctx, (cudaError_t)rc, "plan");
-    ctx->stage_end(HFX_STAGE_WINDOWS, 6, ns);  // k_windows + 5 planning kernels
-    uint32_t ngroups = 0, total_items = 0;
+    ctx->stage_end(HFX_STAGE_WINDOWS, dense_on ? 8 : 6, ns);  // k_windows + the planning kernels
+    uint32_t ngroups = 0, total_items = 0, ntiles = 0, ditems = 0;
     if (ctx->gmode >= 1) {
         // capacities of the graph; a batch that needs more is reported (k_clamp_items)
         ngroups = ctx->cap_groups;
@@ -658,14 +680,37 @@ int32_t search_batched(hfx_ctx *ctx, const hfx_search_params *p, const Batch &b,
         rc = hfx_clamp_groups(ws.ngroups, ngroups, ctx->d_err.as<uint32_t>(), ctx->stream);
         if (!rc)
             rc = hfx_clamp_items(ws.item_off, (int64_t)ns + 1, total_items, ctx->d_err.as<uint32_t>(), ctx->stream);
+        if (!rc && dense_on) {
+            ntiles = ctx->cap_tiles;
+            ditems = ctx->cap_ditems;
+            rc = hfx_clamp_groups(dw.n_tiles, ntiles, ctx->d_err.as<uint32_t>(), ctx->stream);
+            if (!rc)
+                rc = hfx_clamp_items(dw.item_off, (int64_t)dw.cap_blocks + 1, ditems, ctx->d_err.as<uint32_t>(),
+                                     ctx->stream);
+        }
         if (rc) return cuda_fail(ctx, (cudaError_t)rc, "k_clamp_items");
     } else {
-        uint32_t hs[4];
-        HFX_CUDA(cudaMemcpyAsync(hs, scal, 16, cudaMemcpyDeviceToHost, ctx->stream), "D2H plan");
+        uint32_t hs[6];
+        HFX_CUDA(cudaMemcpyAsync(hs, scal, 24, cudaMemcpyDeviceToHost, ctx->stream), "D2H plan");
         HFX_CUDA(cudaStreamSynchronize(ctx->stream), "sync");
         ngroups = hs[1];
         total_items = hs[2];
+        if (dense_on) {
+            ntiles = hs[4];
+            ditems = hs[5];
+        }
         ctx->last_items = total_items;
+        ctx->last_tiles = ntiles;
+        ctx->last_ditems = ditems;
+    }
+    const bool rescore = elem_kind != 0 || ntiles > 0;
+    if (rescore && elem_kind == 0) K = kMaxTopK;
+    const int pieces = hfx_dense_pieces(elem_kind);
+    uint8_t *dtiles = nullptr;
+    if (dense_on && ntiles > 0) {
+        dtiles = ctx->buf<uint8_t>("d_tiles", (size_t)ntiles * dense_tile_bytes(stride, pieces), e);
+        if (!e) dw.left = ctx->buf<unsigned long long>("d_left", (size_t)ditems * kDenseSpectra * kDenseQueue + 1, e);
+        if (e) return cuda_fail(ctx, e, "alloc dense blocks");
     }
     const size_t esz = elem_kind == 0 ? 4 : 2;
     void *tiles = ctx->buf<uint8_t>("tiles", (size_t)ngroups * stride * G * esz + 64, e);
@@ -684,7 +729,11 @@ int32_t search_batched(hfx_ctx *ctx, const hfx_search_params *p, const Batch &b,
     ctx->stage_begin(HFX_STAGE_PACK);
     rc = hfx_pack_tiles(src_rows, elem_kind, stride, meta, ws, tiles, ngroups, G, ctx->stream);
     if (rc) return cuda_fail(ctx, (cudaError_t)rc, "k_pack_tiles");
-    ctx->stage_end(HFX_STAGE_PACK, ngroups > 0 ? 1 : 0, ngroups);
+    if (dtiles) {
+        rc = hfx_dense_pack(rows, stride, ws, dw, ntiles, pieces, dtiles, ctx->d_err.as<uint32_t>(), ctx->stream);
+        if (rc) return cuda_fail(ctx, (cudaError_t)rc, "k_dense_pack");
+    }
+    ctx->stage_end(HFX_STAGE_PACK, (ngroups > 0 ? 1 : 0) + (dtiles ? 1 : 0), ngroups);
     if (!plain_on) {
     } else if (p->batch_mode != 1 && !long_rows) {
         // fused: every work item rebuilds its candidates' ion lists
@@ -760,7 +809,13 @@ int32_t search_batched(hfx_ctx *ctx, const hfx_search_params *p, const Batch &b,
                              elem_kind, stride, wb, we, ws, tiles, G, K, 0, ps, pk, stats,
                              ctx->d_err.as<uint32_t>(), ctx->stream, sink, sink_off);
         if (rc) return cuda_fail(ctx, (cudaError_t)rc, "k_score_lists");
-        ctx->stage_end(HFX_STAGE_SCORE, 1, 0);
+        if (dtiles) {
+            rc = hfx_dense_score((const uint16_t *)lists, total10 * 10, ctx->d_lstart.as<uint32_t>(), total10, llen,
+                                 (uint32_t)ctx->num_pep, dtiles, ntiles, stride, pieces, wb, we, ns, ws, dw, K,
+                                 stats, ctx->d_err.as<uint32_t>(), ctx->stream);
+            if (rc) return cuda_fail(ctx, (cudaError_t)rc, "k_dense_score");
+        }
+        ctx->stage_end(HFX_STAGE_SCORE, dtiles ? 2 : 1, 0);
         if (stats) {
             unsigned long long h[8];
             HFX_CUDA(cudaMemcpyAsync(h, stats, 64, cudaMemcpyDeviceToHost, ctx->stream), "D2H stats");
@@ -848,9 +903,9 @@ int32_t search_batched(hfx_ctx *ctx, const hfx_search_params *p, const Batch &b,
         rc = hfx_merge_with_mods(ps, pk, ws.item_off, ms, mk, mitem_off, ctx->num_mod, ws, meta, ns, G, K, plain_on,
                                  ks, kk, ctx->stream);
     else
-        rc = hfx_batched_merge(ps, pk, ws, meta, ns, G, K, K, ks, kk, ctx->stream);
+        rc = hfx_batched_merge(ps, pk, ws, meta, wb, we, ns, G, K, K, ks, kk, dense_on ? &dw : nullptr, ctx->stream);
     if (rc) return cuda_fail(ctx, (cudaError_t)rc, "k_merge_items");
-    if (elem_kind == 0) {
+    if (!rescore) {
         rc = hfx_finish(ks, kk, ns, p->top_n, ctx->d_idx.as<uint32_t>(), wb, we, meta, out_s, out_k, out_pep,
                         plain_on, ncm, out_ncand, ctx->stream);
         if (rc) return cuda_fail(ctx, (cudaError_t)rc, "k_finish");
@@ -992,6 +1047,8 @@ int32_t search_graph(hfx_ctx *ctx, const hfx_search_params *p, const Batch &b, f
     ctx->cap_stride = ctx->last_stride;
     ctx->cap_groups = (uint32_t)((b.nspec + G - 1) / G + 24);  // <= one partial group per class
     ctx->cap_items = ctx->last_items + ctx->last_items / 4 + 64;
+    ctx->cap_tiles = ctx->last_tiles ? ctx->last_tiles + ctx->last_tiles / 4 + 2 : 0;
+    ctx->cap_ditems = ctx->last_ditems ? ctx->last_ditems + ctx->last_ditems / 4 + 64 : 0;
     ctx->cap_mitems = ctx->last_mitems + ctx->last_mitems / 4 + 64;
     ctx->cap_iso = ctx->last_iso + ctx->last_iso / 4 + 64;
     ctx->cap_iso_entries = ctx->last_iso_entries + ctx->last_iso_entries / 4 + 4096;
@@ -1534,7 +1591,7 @@ int32_t hfx_search_evalues(hfx_ctx *ctx, const hfx_search_params *p, const float
     ws.group_of = ctx->buf<int32_t>("b_groupof", ns, e);
     ws.slot_of = ctx->buf<int32_t>("b_slotof", ns, e);
     if (e) return cuda_fail(ctx, e, "alloc");
-    rc = hfx_batched_plan(meta, ns, wb, we, G, chunk, p->chunk > 0 ? 0 : 1, ws, ctx->stream);
+    rc = hfx_batched_plan(meta, ns, wb, we, G, chunk, p->chunk > 0 ? 0 : 1, ws, nullptr, ctx->stream);
     if (rc) return cuda_fail(ctx, (cudaError_t)rc, "plan");
     uint32_t hs[4];
     HFX_CUDA(cudaMemcpyAsync(hs, scal, 16, cudaMemcpyDeviceToHost, ctx->stream), "D2H plan");

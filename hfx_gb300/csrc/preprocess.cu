@@ -73,6 +73,7 @@ __global__ void k_layout(const float *__restrict__ mz, const int64_t *__restrict
     int32_t ch = (rr >= 1.0f) ? (rr > 1000.0f ? 1000 : (int32_t)rr) : 0;
     m.charges_plain = (ch >= 1 && ch <= 4) ? ch : 0;
     m.charges_mod = (ch >= 1 && ch <= 10) ? min(ch, 4) : 0;  // mion_series.cu:303-306, 425-438
+    m.nonfinite = 0;
     meta[s] = m;
     if (m.status == 0) atomicMax(max_len, (uint32_t)m.len);
 }
@@ -108,7 +109,7 @@ __device__ __forceinline__ int32_t block_excl_scan(int32_t v, int32_t *warp_tot,
 __global__ void __launch_bounds__(256) k_preprocess(const float *__restrict__ mz, const float *__restrict__ it,
                                                     const int64_t *__restrict__ off,
                                                     const float *__restrict__ pcr, LayoutParams lp,
-                                                    const SpecMeta *__restrict__ meta, int64_t stride,
+                                                    SpecMeta *__restrict__ meta, int64_t stride,
                                                     float *__restrict__ out32, __nv_bfloat16 *__restrict__ outbf,
                                                     __half *__restrict__ outh, int fold_nonzero) {
     extern __shared__ float sh[];
@@ -142,6 +143,7 @@ __global__ void __launch_bounds__(256) k_preprocess(const float *__restrict__ mz
         if (!(q >= 0.0f) || q >= (float)len) continue;  // the reference raises here
         const float v = __fsqrt_rn(it[o0 + i]);
         if (v >= 0.0f) atomicMax((int *)&e[(int32_t)q], __float_as_int(v));
+        if (isinf(v)) meta[s].nonfinite = 1;
     }
     __syncthreads();
     // normaliseByRegion, Correlation.hs:84-96
@@ -385,7 +387,7 @@ int hfx_launch_layout(const float *mz, const int64_t *off, const float *pcr, con
 }
 
 int hfx_launch_preprocess(const float *mz, const float *it, const int64_t *off, const float *pcr,
-                          const LayoutParams &lp, const SpecMeta *meta, int32_t nspec, int64_t stride,
+                          const LayoutParams &lp, SpecMeta *meta, int32_t nspec, int64_t stride,
                           float *out32, __nv_bfloat16 *outbf, __half *outh, uint32_t *err, cudaStream_t st) {
     if (nspec <= 0) return 0;
     size_t smem = (size_t)stride * sizeof(float);
