@@ -151,7 +151,7 @@ __device__ __forceinline__ float residue_mass(float mt_lane, uint32_t byte) {
 // chunk in peptide order: returns the mass to add to this lane's residue
 // (0 = unmodified).  `valid` is false for lanes past the peptide's end.
 struct NoMods {
-    __device__ __forceinline__ float chunk_add(uint32_t /*byte*/, bool /*valid*/) { return 0.0f; }
+    __device__ __forceinline__ float chunk_add(uint32_t /*byte*/, bool /*valid*/, int /*lane*/ = 0) { return 0.0f; }
 };
 
 // Words [lo, hi) of the bit planes that hold set bits.

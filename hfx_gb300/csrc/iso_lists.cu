@@ -241,12 +241,13 @@ __global__ void __launch_bounds__(256) k_iso_positions(DevDB db, DevMods mods, c
     append_work(wl, cls, t);
 }
 
-// 4b. one warp per isoform: the distinct-bin list of every needed level
+// 4b. class_lanes lanes per isoform: the distinct-bin list of every needed level
 // (build_lists; classes as in k_gen_lists).  The 3.93 M lists (1.17 G
 // entries) of 1,000 spectra against 5,000 proteins: 5.57 ms by bit planes,
-// 4.15 ms by rank.
-template <bool FastDiv, int NC>
-__global__ void __launch_bounds__(256, NC == 0 ? 1 : 4) k_gen_iso_lists(DevDB db, DevMods mods, const int32_t *__restrict__ cover,
+// 4.15 ms by rank; two short ladders a warp took 0.48 ms off the 5.11 ms of
+// all launches that prepare those isoforms.
+template <bool FastDiv, int kClass>
+__global__ void __launch_bounds__(256, kClass == 0 ? 1 : 4) k_gen_iso_lists(DevDB db, DevMods mods, const int32_t *__restrict__ cover,
                                                        int64_t npep1, int32_t nbins,
                                                        const uint32_t *__restrict__ lstart,
                                                        const uint64_t *__restrict__ iso_key,
@@ -257,34 +258,38 @@ __global__ void __launch_bounds__(256, NC == 0 ? 1 : 4) k_gen_iso_lists(DevDB db
                                                        WorkLists wl, unsigned long long *__restrict__ stats,
                                                        uint32_t *__restrict__ err) {
     extern __shared__ __align__(128) uint8_t smem[];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const RankBufs rb = rank_bufs(smem + (size_t)warp * rank_bytes(nbins), nbins);
-    for (int32_t i = lane; i < (rb.words >> 1); i += 32) sts_u128(rb.pl + 16u * i, make_uint4(0u, 0u, 0u, 0u));
+    constexpr int W = class_lanes(kClass);
+    const int lane = threadIdx.x & (W - 1), nw = blockDim.x / W;
+    const RankBufs rb = rank_bufs(smem + (size_t)(threadIdx.x / W) * rank_bytes(nbins, kClass), nbins, kClass);
+    for (int32_t i = lane; i < (rb.words >> 1); i += W) sts_u128(rb.pl + 16u * i, make_uint4(0u, 0u, 0u, 0u));
     __syncwarp();
-    const float mt_lane = db.mt[lane];
+    const float mt_lane = db.mt[threadIdx.x & 31];
     float ma_lane = 0.0f;
 #pragma unroll
     for (int i = 0; i < kMaxMa; ++i)
-        if (lane == i && i < mods.num_ma) ma_lane = mods.ma_mass[i];
-    const uint32_t total = wl.count(NC);
-    const uint32_t *work = wl.list(NC);
+        if ((int)(threadIdx.x & 31) == i && i < mods.num_ma) ma_lane = mods.ma_mass[i];
+    const uint32_t total = wl.count(kClass);
+    const uint32_t *work = wl.list(kClass);
     // per-warp work counters (a warp's share of one launch fits 32 bits)
     uint32_t my_lists = 0, my_entries = 0, my_iso = 0, my_res = 0;
-    for (uint32_t i = blockIdx.x * nw + warp; i < total; i += gridDim.x * nw) {
-        const uint32_t t = work[i];
+    for (uint32_t i = blockIdx.x * nw + threadIdx.x / W; (i & ~(32u / W - 1u)) < total; i += gridDim.x * nw) {
+        // (a warp's last isoform may have no partner: no levels, no prefixes)
+        const bool have = i < total;
+        const uint32_t t = work[have ? i : i - 1u];
         const uint64_t key = iso_key[t];
         const int32_t mu = (int32_t)((key >> 54) & 0x1FFu);
         const uint32_t p = (uint32_t)((key >> 27) & 0x7FFFFFFu);
-        const uint32_t need = need_levels(cover, npep1, mu, p);
+        uint32_t need = have ? need_levels(cover, npep1, mu, p) : 0u;
         const int zmax = 32 - __clz(need);
-        const uint32_t tc = db.tc_sorted[p], tn = db.tn_sorted[p];
+        const uint32_t tc = db.tc_sorted[p];
+        uint32_t tn = need ? db.tn_sorted[p] : tc;
         const uint32_t unit = lstart[p + 1] - lstart[p];
         const uint64_t off = iso_off[t];
-        if (off + iso_slot(unit, zmax) > list_total ||
-            (tn > tc && (int64_t)(tn - tc) > 32ll * pos_words)) {  // neither happens for an expanded record
+        if (need && (off + iso_slot(unit, zmax) > list_total ||
+                     (tn > tc && (int64_t)(tn - tc) > 32ll * pos_words))) {  // neither happens for an expanded record
             if (lane == 0) atomicOr(err, kErrBounds);
-            if (lane < kLevels) iso_len[(size_t)t * kLevels + lane] = 0;
-            continue;
+            need = 0u;
+            tn = tc;
         }
         // the residues this isoform modifies (k_iso_positions)
         const ModPositions iso{iso_pos + (size_t)t * pos_words, ma_lane, 0u};
@@ -292,14 +297,14 @@ __global__ void __launch_bounds__(256, NC == 0 ? 1 : 4) k_gen_iso_lists(DevDB db
         const float residual = __fadd_rn(db.r_sorted[p], mods.delta[mu]);
         // every level up to zmax has its place in the slot, unit z >= 10 (tn - tc) z entries
         const ListSlots ls{lists + off, unit, 0ull, iso_len + (size_t)t * kLevels, 1ull};
-        const int entries = build_lists<FastDiv, NC>(rb, db.ions, tc, tn, residual, need, (uint32_t)nbins, mt_lane,
-                                                     iso, ls);
-        if (lane < kLevels && !((need >> lane) & 1u)) iso_len[(size_t)t * kLevels + lane] = 0;
+        const int entries = build_lists<FastDiv, kClass>(rb, db.ions, tc, tn, residual, need, (uint32_t)nbins,
+                                                         mt_lane, iso, ls);
+        if (have && lane < kLevels && !((need >> lane) & 1u)) iso_len[(size_t)t * kLevels + lane] = 0;
         if (entries < 0) {
-            if (lane == 0) wl.list(0)[atomicAdd(wl.w, 1u)] = t;
+            if (lane == 0 && need) wl.list(0)[atomicAdd(wl.w, 1u)] = t;
             continue;
         }
-        my_iso += 1u;
+        my_iso += have ? 1u : 0u;
         my_res += tn > tc ? tn - tc : 0u;
         my_entries += (uint32_t)entries;
         my_lists += (uint32_t)__popc(need);
@@ -557,8 +562,6 @@ int hfx_iso_generate(const DevDB &db, const DevMods &m, const int32_t *cover, in
                      uint32_t *iso_pos, uint32_t *work, int fastdiv, unsigned long long *stats, uint32_t *err,
                      cudaStream_t st) {
     if (cap_iso == 0) return 0;
-    const int nw = 8;
-    const size_t smem = (size_t)nw * rank_bytes(nbins);
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -566,17 +569,19 @@ int hfx_iso_generate(const DevDB &db, const DevMods &m, const int32_t *cover, in
     cudaMemsetAsync(work, 0, 16, st);
     k_iso_positions<<<(unsigned)(((uint64_t)cap_iso + 255) / 256), 256, 0, st>>>(
         db, m, total_p, cap_iso, iso_key, pos_words, iso_pos, wl, iso_len, err);
-    auto run = [&](auto f, int most) {
+    auto run = [&](auto f, int cls) {
+        const size_t smem = (size_t)(256 / class_lanes(cls)) * rank_bytes(nbins, cls);
         cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         int per = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, f, nw * 32, smem);
-        f<<<sms * std::max(1, std::min(per, most)), nw * 32, smem, st>>>(
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, f, 256, smem);
+        f<<<sms * std::max(1, cls ? per : std::min(per, 2)), 256, smem, st>>>(
             db, m, cover, (int64_t)db.num_pep + 1, nbins, lstart, iso_key, iso_off, lists, list_total, iso_len,
             pos_words, iso_pos, wl, stats, err);
     };
-    run(fastdiv ? k_gen_iso_lists<true, 1> : k_gen_iso_lists<false, 1>, 32);
-    run(fastdiv ? k_gen_iso_lists<true, 2> : k_gen_iso_lists<false, 2>, 32);
-    run(fastdiv ? k_gen_iso_lists<true, 0> : k_gen_iso_lists<false, 0>, 2);
+    run(fastdiv ? k_gen_iso_lists<true, 3> : k_gen_iso_lists<false, 3>, 3);
+    run(fastdiv ? k_gen_iso_lists<true, 1> : k_gen_iso_lists<false, 1>, 1);
+    run(fastdiv ? k_gen_iso_lists<true, 2> : k_gen_iso_lists<false, 2>, 2);
+    run(fastdiv ? k_gen_iso_lists<true, 0> : k_gen_iso_lists<false, 0>, 0);
     return (int)cudaGetLastError();
 }
 

@@ -73,39 +73,41 @@ __global__ void __launch_bounds__(256) k_list_work(DevDB db, const int32_t *__re
     append_work(wl, cls, p | need << kNeedShift);
 }
 
-// One warp per needed candidate peptide of class NC: the sorted distinct-bin
-// list of every needed charge level (build_lists: the level-z list carries the
+// The sorted distinct-bin list of every needed charge level of the candidates of
+// one class, class_lanes lanes each (build_lists: the level-z list carries the
 // level-(z-1) list over and adds the charge-z ions).  The 3.84 M lists (946 M
 // entries) of 10,000 spectra against 20,000 proteins, coverage and work lists
-// included: 4.12 ms by bit planes and a bit loop, 2.51 ms by rank; issue 70 %
-// of the slots, shared memory 50 % of its wavefronts.
-template <bool FastDiv, int NC>
-__global__ void __launch_bounds__(256, NC == 0 ? 1 : 4) k_gen_lists(DevDB db, int32_t nbins,
-                                                                    const uint32_t *__restrict__ lstart,
-                                                                    uint64_t total10, uint16_t *__restrict__ lists,
-                                                                    uint16_t *__restrict__ list_len, WorkLists wl,
-                                                                    unsigned long long *__restrict__ stats) {
+// included: 4.12 ms by bit planes and a bit loop, 2.48 ms by rank with a warp each,
+// 1.98 ms with two short ladders a warp.
+template <bool FastDiv, int kClass>
+__global__ void __launch_bounds__(256, kClass == 0 ? 1 : 4) k_gen_lists(DevDB db, int32_t nbins,
+                                                                        const uint32_t *__restrict__ lstart,
+                                                                        uint64_t total10, uint16_t *__restrict__ lists,
+                                                                        uint16_t *__restrict__ list_len, WorkLists wl,
+                                                                        unsigned long long *__restrict__ stats) {
     extern __shared__ __align__(128) uint8_t smem[];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const RankBufs rb = rank_bufs(smem + (size_t)warp * rank_bytes(nbins), nbins);
+    constexpr int W = class_lanes(kClass);
+    const int lane = threadIdx.x & (W - 1), nw = blockDim.x / W;
+    const RankBufs rb = rank_bufs(smem + (size_t)(threadIdx.x / W) * rank_bytes(nbins, kClass), nbins, kClass);
     __shared__ unsigned long long s_stats[3];
     if (threadIdx.x < 3) s_stats[threadIdx.x] = 0ull;
-    for (int32_t i = lane; i < (rb.words >> 1); i += 32) sts_u128(rb.pl + 16u * i, make_uint4(0u, 0u, 0u, 0u));
+    for (int32_t i = lane; i < (rb.words >> 1); i += W) sts_u128(rb.pl + 16u * i, make_uint4(0u, 0u, 0u, 0u));
     __syncthreads();
-    const float mt_lane = db.mt[lane];
-    const uint32_t total = wl.count(NC);
-    const uint32_t *work = wl.list(NC);
+    const float mt_lane = db.mt[threadIdx.x & 31];
+    const uint32_t total = wl.count(kClass);
+    const uint32_t *work = wl.list(kClass);
     uint32_t my_lists = 0, my_entries = 0, my_res = 0;
-    for (uint32_t t = blockIdx.x * nw + warp; t < total; t += gridDim.x * nw) {
-        const uint32_t w = work[t];
+    for (uint32_t t = blockIdx.x * nw + threadIdx.x / W; (t & ~(32u / W - 1u)) < total; t += gridDim.x * nw) {
+        // (a warp's last candidate may have no partner: no levels, no prefixes)
+        const uint32_t w = t < total ? work[t] : 0u;
         const uint32_t p = w & ((1u << kNeedShift) - 1u), need = w >> kNeedShift;
-        const uint32_t tc = db.tc_sorted[p], tn = db.tn_sorted[p];
+        const uint32_t tc = db.tc_sorted[p], tn = need ? db.tn_sorted[p] : tc;
         // the slot holds 10 (tn - tc) z entries or more: every list fits
         const ListSlots ls{lists, total10, lstart[p], list_len + p, db.num_pep};
-        const int entries = build_lists<FastDiv, NC>(rb, db.ions, tc, tn, db.r_sorted[p], need, (uint32_t)nbins,
-                                                     mt_lane, NoMods{}, ls);
+        const int entries = build_lists<FastDiv, kClass>(rb, db.ions, tc, tn, db.r_sorted[p], need, (uint32_t)nbins,
+                                                         mt_lane, NoMods{}, ls);
         if (entries < 0) {
-            if (lane == 0) wl.list(0)[atomicAdd(wl.w, 1u)] = w;
+            if (lane == 0 && need) wl.list(0)[atomicAdd(wl.w, 1u)] = w;
             continue;
         }
         my_entries += (uint32_t)entries;
@@ -732,24 +734,24 @@ size_t hfx_lists_work_words(uint64_t n) { return work_words(n); }
 int hfx_lists_generate(const DevDB &db, const int32_t *cover, int64_t npep1, int32_t nbins, const uint32_t *lstart,
                        uint64_t total10, uint16_t *lists, uint16_t *list_len, uint32_t *work, int fastdiv,
                        unsigned long long *stats, cudaStream_t st) {
-    const int nw = 8;
-    const size_t smem = (size_t)nw * rank_bytes(nbins);
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const WorkLists wl{work, db.num_pep};
     cudaMemsetAsync(work, 0, 16, st);
     k_list_work<false><<<(db.num_pep + 255) / 256, 256, 0, st>>>(db, cover, npep1, list_len, wl, nullptr);
-    auto run = [&](auto f, int most) {
+    auto run = [&](auto f, int cls) {
+        const size_t smem = (size_t)(256 / class_lanes(cls)) * rank_bytes(nbins, cls);
         cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         int per = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, f, nw * 32, smem);
-        f<<<sms * std::max(1, std::min(per, most)), nw * 32, smem, st>>>(db, nbins, lstart, total10, lists, list_len,
-                                                                         wl, stats);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, f, 256, smem);
+        f<<<sms * std::max(1, cls ? per : std::min(per, 2)), 256, smem, st>>>(db, nbins, lstart, total10, lists,
+                                                                             list_len, wl, stats);
     };
-    run(fastdiv ? k_gen_lists<true, 1> : k_gen_lists<false, 1>, 32);
-    run(fastdiv ? k_gen_lists<true, 2> : k_gen_lists<false, 2>, 32);
-    run(fastdiv ? k_gen_lists<true, 0> : k_gen_lists<false, 0>, 2);
+    run(fastdiv ? k_gen_lists<true, 3> : k_gen_lists<false, 3>, 3);
+    run(fastdiv ? k_gen_lists<true, 1> : k_gen_lists<false, 1>, 1);
+    run(fastdiv ? k_gen_lists<true, 2> : k_gen_lists<false, 2>, 2);
+    run(fastdiv ? k_gen_lists<true, 0> : k_gen_lists<false, 0>, 0);
     return (int)cudaGetLastError();
 }
 

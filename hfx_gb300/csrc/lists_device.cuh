@@ -43,16 +43,22 @@ constexpr int kStageCap = 1024;
 // have bits of their own (0, 1 and nbins + 2 .. nbins + 4) and marking needs no
 // test; rank_scan drops those.
 __host__ __device__ __forceinline__ int32_t rank_words(int32_t nbins) { return (((nbins + 2) >> 5) + 3) & ~1; }
-// Shared memory of one warp (a multiple of 16 bytes).
-__host__ __device__ __forceinline__ size_t rank_bytes(int32_t nbins) {
-    return (size_t)rank_words(nbins) * 8 + (size_t)2 * kStageCap * 2;
+// Lanes that hold a candidate of a class, and its staging room: a ladder of up
+// to 16 prefixes takes half a warp.  The generators are bound by instructions
+// issued per warp, and the mean ladder has 16 prefixes: one candidate a warp
+// left half its lanes idle.
+__host__ __device__ constexpr int class_lanes(int cls) { return cls == 3 ? 16 : 32; }
+__host__ __device__ constexpr int class_cap(int cls) { return cls == 3 ? 640 : kStageCap; }  // 640 = 16 prefixes x 4 charges x 10
+// Shared memory of one candidate (a multiple of 16 bytes).
+__host__ __device__ __forceinline__ size_t rank_bytes(int32_t nbins, int cls) {
+    return (size_t)rank_words(nbins) * 8 + (size_t)2 * class_cap(cls) * 2;
 }
-__device__ __forceinline__ RankBufs rank_bufs(const uint8_t *base, int32_t nbins) {
+__device__ __forceinline__ RankBufs rank_bufs(const uint8_t *base, int32_t nbins, int cls) {
     RankBufs rb;
     rb.words = rank_words(nbins);
     rb.pl = smem_u32(base);
     rb.a = rb.pl + (uint32_t)rb.words * 8u;
-    rb.b = rb.a + kStageCap * 2u;
+    rb.b = rb.a + (uint32_t)class_cap(cls) * 2u;
     return rb;
 }
 
@@ -131,22 +137,23 @@ struct ListSlots {
     }
 };
 
-// The b-ladder of residues [base, base + cnt), cnt <= 32, after `carry`: the
-// reference warp scan (ion_series.cu:25-56, 176-213), lane i prefix i.
-template <typename Mods>
+// The b-ladder of residues [base, base + cnt), cnt <= W, after `carry`: the
+// reference warp scan (ion_series.cu:25-56, 176-213), lane i of the W prefix i
+// (for 16 its last stride moves nothing).
+template <int W = 32, typename Mods>
 __device__ __forceinline__ float ladder_chunk(const uint8_t *__restrict__ ions, uint32_t base, int cnt,
                                               float mt_lane, Mods &mods, float carry) {
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & (W - 1);
     uint32_t byte = 0;
     if (lane < cnt) byte = __ldg(ions + base + lane);
     float v = residue_mass(mt_lane, byte);
-    const float add = mods.chunk_add(byte, lane < cnt);
+    const float add = mods.chunk_add(byte, lane < cnt, lane);
     if (add != 0.0f) v = __fadd_rn(v, add);
     if (lane >= cnt) v = 0.0f;
     if (lane == 0) v = __fadd_rn(v, carry);
 #pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const float t = __shfl_up_sync(kFullMask, v, d);
+    for (int d = 1; d < W; d <<= 1) {
+        const float t = __shfl_up_sync(kFullMask, v, d, W);
         if (lane >= d) v = __fadd_rn(v, t);
     }
     return v;
@@ -222,8 +229,9 @@ __device__ __forceinline__ void mark_item(uint32_t pl, const ItemBits &t, uint32
 // `words` words; returns the number of set bits.  A lane takes two
 // neighbouring words, 16 bytes: free of bank conflicts (four words a lane in
 // two accesses took eight wavefronts each, 40 % of the kernel's).
+template <int W = 32>
 __device__ __forceinline__ int rank_scan(uint32_t pl, int32_t words, uint32_t nbins) {
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & (W - 1);
     if (lane < 3) {
         const uint32_t top = nbins + 2u;
         const uint32_t at = lane == 0 ? pl : word_addr(pl, top) + (lane == 2 ? 8u : 0u);
@@ -233,17 +241,22 @@ __device__ __forceinline__ int rank_scan(uint32_t pl, int32_t words, uint32_t nb
     __syncwarp();
     int before = 0;
 #pragma unroll 1
-    for (int w0 = 0; w0 < words; w0 += 64) {
+    for (int w0 = 0; w0 < words; w0 += 2 * W) {
         const int w = w0 + 2 * lane;
         const uint32_t at = pl + 8u * (uint32_t)w;
         uint4 u = make_uint4(0u, 0u, 0u, 0u);
         if (w < words) u = lds_u128(at);
         const int c0 = __popc(u.x), c1 = c0 + __popc(u.z);
-        const int incl = warp_incl_scan(c1);
+        int incl = c1;
+#pragma unroll
+        for (int d = 1; d < W; d <<= 1) {
+            const int t = __shfl_up_sync(kFullMask, incl, d, W);
+            if (lane >= d) incl += t;
+        }
         u.y = (uint32_t)(before + incl - c1);
         u.w = u.y + (uint32_t)c0;
         if (w < words) sts_u128(at, u);
-        before += __shfl_sync(kFullMask, incl, 31);
+        before += __shfl_sync(kFullMask, incl, W - 1, W);
     }
     __syncwarp();
     return before;
@@ -255,32 +268,33 @@ __device__ __forceinline__ uint32_t rank_in(uint2 e, uint32_t bit) {
 }
 __device__ __forceinline__ uint32_t rank_of(uint32_t pl, uint32_t bit) { return rank_in(lds_u64(word_addr(pl, bit)), bit); }
 
-// The level lists of one candidate with up to 32 NC prefixes (NC = 1 or 2),
-// its ladder and the level's bins kept in registers between marking and
-// placing.  `need`: bit z - 1 asks for the level-z list.  Returns the entries
+// The level lists of one candidate with up to W NC prefixes (NC = 1 or 2), held
+// by W lanes (two candidates a warp for 16: the warp-wide steps are common to
+// both, and the levels go up to the higher one's), its ladder and the level's
+// bins kept in registers between marking and placing.  `need`: bit z - 1 asks for the level-z list.  Returns the entries
 // written, or -1 when a list does not fit the staging buffers (or a mass is
 // out of `quotient`'s range).  The bits are left cleared.
-template <bool FastDiv, int NC, typename Mods>
+template <bool FastDiv, int NC, int W, typename Mods>
 __device__ __forceinline__ int build_lists_staged(const RankBufs &rb, const uint8_t *__restrict__ ions, uint32_t tc,
                                                   int len, float residual, uint32_t need, uint32_t nbins,
                                                   float mt_lane, Mods mods, const ListSlots &ls) {
-    const int lane = threadIdx.x & 31;
-    const int zmax = 32 - __clz(need);
+    const int lane = threadIdx.x & (W - 1);
+    const int zmax = 32 - __clz(__reduce_or_sync(kFullMask, need));  // of the warp's candidates
     const uint32_t pl = rb.pl;
     float v[NC], y[NC];
     float carry = 0.0f, top = 0.0f;
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
-        v[c] = ladder_chunk(ions, tc + 32u * c, min(32, len - 32 * c), mt_lane, mods, carry);
-        if (c + 1 < NC) carry = __shfl_sync(kFullMask, v[c], 31);
+        v[c] = ladder_chunk<W>(ions, tc + (uint32_t)(W * c), min(W, len - W * c), mt_lane, mods, carry);
+        if (c + 1 < NC) carry = __shfl_sync(kFullMask, v[c], W - 1, W);
         y[c] = __fsub_rn(residual, v[c]);
         // lanes past the end: ions past every row, which nothing below marks or writes
-        if (lane + 32 * c < len) top = fmaxf(top, fmaxf(v[c], y[c]));
+        if (lane + W * c < len) top = fmaxf(top, fmaxf(v[c], y[c]));
         else v[c] = y[c] = 0x1p21f;
     }
     // no ion lies above its prefix or suffix mass + H2O + H: the words in use
     const uint32_t hi = __reduce_max_sync(kFullMask, __float2uint_rz(__fadd_rn(top, 24.0f)));
-    if (hi >= (1u << 21)) return -1;
+    if (hi >= (1u << 21)) return -1;  // (either candidate's: both are left)
     const int32_t words = rank_words((int32_t)min(hi, nbins));
     uint32_t dst = rb.a, prev = rb.b;
     int n_prev = 0, entries = 0;
@@ -299,14 +313,14 @@ __device__ __forceinline__ int build_lists_staged(const RankBufs &rb, const uint
             mark_item(pl, t[c], nbins);
         }
         __syncwarp();
-        const int n = rank_scan(pl, words, nbins);
-        if (n > kStageCap) {
+        const int n = rank_scan<W>(pl, words, nbins);
+        if (W == 32 && n > kStageCap) {  // (16 prefixes' lists always fit)
             entries = -1;
             break;
         }
         // entries that are not carried over read as no level
 #pragma unroll 1
-        for (int i = lane; i < ((n + 7) >> 3); i += 32) sts_u128(dst + 16u * i, make_uint4(0u, 0u, 0u, 0u));
+        for (int i = lane; i < ((n + 7) >> 3); i += W) sts_u128(dst + 16u * i, make_uint4(0u, 0u, 0u, 0u));
         __syncwarp();
         // level 1 (10); bit s is bin s - 2
 #pragma unroll
@@ -321,7 +335,7 @@ __device__ __forceinline__ int build_lists_staged(const RankBufs &rb, const uint
         __syncwarp();
         // the previous level's list at its new places, two entries a lane
 #pragma unroll 1
-        for (int i = 2 * lane; i < n_prev; i += 64) {
+        for (int i = 2 * lane; i < n_prev; i += 2 * W) {
             const uint32_t p = lds_u32(prev + 2u * i);
             const uint32_t s0 = ((p & 0xFFFFu) >> 2) + 2u, s1 = i + 1 < n_prev ? (p >> 18) + 2u : 0u;
             const uint2 e0 = lds_u64(word_addr(pl, s0)), e1 = lds_u64(word_addr(pl, s1));
@@ -363,7 +377,7 @@ __device__ __forceinline__ int build_lists_staged(const RankBufs &rb, const uint
             // boundaries and hold n rounded up to 8 entries
             uint4 *out = reinterpret_cast<uint4 *>(ls.slot(z));
 #pragma unroll 1
-            for (int i = lane; i < ((n + 7) >> 3); i += 32) out[i] = lds_u128(dst + 16u * i);
+            for (int i = lane; i < ((n + 7) >> 3); i += W) out[i] = lds_u128(dst + 16u * i);
             if (lane == 0) ls.len[(uint64_t)(z - 1) * ls.len_step] = (uint16_t)n;
             entries += n;
         }
@@ -373,7 +387,7 @@ __device__ __forceinline__ int build_lists_staged(const RankBufs &rb, const uint
         prev = swap;
     }
 #pragma unroll 1
-    for (int i = lane; i < (words >> 1); i += 32) sts_u128(pl + 16u * i, make_uint4(0u, 0u, 0u, 0u));
+    for (int i = lane; i < (words >> 1); i += W) sts_u128(pl + 16u * i, make_uint4(0u, 0u, 0u, 0u));
     __syncwarp();
     return entries;
 }
@@ -448,22 +462,23 @@ __device__ __forceinline__ int build_lists_direct(const RankBufs &rb, const uint
     return entries;
 }
 
-// The kernel a candidate's lists are built by: class 1 and 2 hold ladders of
-// up to 32 and 64 prefixes in registers (kept apart because two chunks cost
-// every candidate spills), class 0 is the rest (build_lists_direct).
+// The kernel a candidate's lists are built by: class 3 holds ladders of up to 16
+// prefixes, two a warp, class 1 and 2 ladders of up to 32 and 64 (kept apart
+// because two chunks cost every candidate spills), class 0 is the rest
+// (build_lists_direct).
 __device__ __forceinline__ int list_class(uint32_t tc, uint32_t tn) {
     const uint32_t len = tn > tc ? tn - tc : 0u;
-    return len <= 32u ? 1 : (len <= 64u ? 2 : 0);
+    return len <= 16u ? 3 : (len <= 32u ? 1 : (len <= 64u ? 2 : 0));
 }
 
-// Work lists of the three classes: counts at w[0..2], then `cap` entries each.
+// Work lists of the four classes: counts at w[0..3], then `cap` entries each.
 struct WorkLists {
     uint32_t *w;
     uint64_t cap;
     __device__ __forceinline__ uint32_t count(int c) const { return w[c]; }
     __device__ __forceinline__ uint32_t *list(int c) const { return w + 4 + (uint64_t)c * cap; }
 };
-constexpr int kWorkLists = 3;
+constexpr int kWorkLists = 4;
 __host__ __device__ __forceinline__ size_t work_words(uint64_t cap) { return 4 + kWorkLists * (size_t)cap; }
 
 // Appends `value` to list `cls` (none when negative); every thread of the
@@ -488,17 +503,18 @@ __device__ __forceinline__ void append_work(const WorkLists &wl, int cls, uint32
     if (cls >= 0) wl.list(cls)[s_base[cls] + at] = value;
 }
 
-// All needed level lists of one candidate of class NC: the entries written, or
+// All needed level lists of one candidate of the class: the entries written, or
 // -1 when it is one for class 0 after all.
-template <bool FastDiv, int NC, typename Mods>
+template <bool FastDiv, int kClass, typename Mods>
 __device__ __forceinline__ int build_lists(const RankBufs &rb, const uint8_t *__restrict__ ions, uint32_t tc,
                                            uint32_t tn, float residual, uint32_t need, uint32_t nbins, float mt_lane,
                                            const Mods &mods, const ListSlots &ls) {
     const int len = tn > tc ? (int)(tn - tc) : 0;
-    if constexpr (NC == 0)
+    if constexpr (kClass == 0)
         return build_lists_direct<FastDiv>(rb, ions, tc, len, residual, need, nbins, mt_lane, mods, ls);
     else
-        return build_lists_staged<FastDiv, NC>(rb, ions, tc, len, residual, need, nbins, mt_lane, mods, ls);
+        return build_lists_staged<FastDiv, kClass == 2 ? 2 : 1, class_lanes(kClass)>(rb, ions, tc, len, residual, need,
+                                                                                    nbins, mt_lane, mods, ls);
 }
 
 // Offset of the list of (level z, mass-order position p): every level has a

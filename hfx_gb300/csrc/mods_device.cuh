@@ -180,8 +180,8 @@ struct ModPositions {
     float ma_lane;
     uint32_t c;
 
-    __device__ __forceinline__ float chunk_add(uint32_t byte, bool valid) {
-        const int lane = threadIdx.x & 31;
+    // lane: the residue's place in its chunk
+    __device__ __forceinline__ float chunk_add(uint32_t byte, bool valid, int lane) {
         const uint32_t w = bits[c++];
         const uint32_t t = (byte >> 5) & 7u;
         const float add = __shfl_sync(kFullMask, ma_lane, (int)((t + 7u) & 7u));

@@ -87,3 +87,29 @@ def test_long_row_lists_at_their_edges(gpulib, oracle, width, custom):
     assert np.array_equal(res.key, key)
     assert np.array_equal(res.score.view(np.uint32), sc.view(np.uint32))
     eng.close()
+
+
+@pytest.mark.parametrize("lengths", [[1], [16], [9, 16, 16], [16, 17, 3, 33, 12]])
+def test_short_ladders_share_a_warp(gpulib, oracle, lengths):
+    """Ladders of up to 16 prefixes are built two a warp: odd counts (the last
+    one alone), neighbours that need different levels, 16 against 17."""
+    import hfx_gb300
+    seq, _, _, _, mt = _database(3)
+    tc = np.array([40 * i for i in range(len(lengths))], np.uint32)
+    tn = tc + np.array(lengths, np.uint32)
+    r = np.array([mt[seq[a:b] - 65].astype(np.float64).sum() for a, b in zip(tc, tn)], np.float32)
+    eng = hfx_gb300.Engine(0)
+    eng.upload_db(seq, r, tc, tn, mt)
+    rs, tcs, tns, idx, _ = eng.db_export()
+    parts = [_spectra(20 * c + 1, c, 1500.0) for c in (2, 3, 5)]
+    off = np.concatenate([[0], np.cumsum(np.concatenate([np.diff(p.off) for p in parts]))]).astype(np.int64)
+    sp = synth.Spectra(*(np.concatenate([getattr(p, f) for p in parts]) for f in ("mz", "it")), off,
+                       *(np.concatenate([getattr(p, f) for p in parts]) for f in ("pcr", "z", "tol")))
+    # charge 2 reaches every peptide; 3 and 5 only those around their own mass
+    sp.tol[6:] = 300.0
+    res = eng.search(sp, hfx_gb300.default_params(top_n=8, batch_mode=1))
+    sc, _, key, pep, nc = oracle.search(oracle.pack_ions(seq), mt, rs, tcs, tns, idx, sp, topn=8)
+    assert np.array_equal(res.ncand, nc)
+    assert np.array_equal(res.key, key)
+    assert np.array_equal(res.score.view(np.uint32), sc.view(np.uint32))
+    eng.close()
