@@ -63,7 +63,8 @@ enum : uint32_t {
 
 int hfx_launch_layout(const float *mz, const int64_t *off, const float *pcr, const float *z,
                       const float *tol, int32_t nspec, const hfx::LayoutParams &lp,
-                      hfx::SpecMeta *meta, uint32_t *max_len, uint32_t *err, cudaStream_t st);
+                      hfx::SpecMeta *meta, uint32_t *max_len, uint32_t *err, cudaStream_t st,
+                      int32_t *lens = nullptr, float *masses = nullptr);
 int hfx_launch_preprocess(const float *mz, const float *it, const int64_t *off, const float *pcr,
                           const hfx::LayoutParams &lp, hfx::SpecMeta *meta, int32_t nspec,
                           int64_t stride, float *out32, __nv_bfloat16 *outbf, __half *outh, uint32_t *err,

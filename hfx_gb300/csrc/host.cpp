@@ -1943,27 +1943,14 @@ int32_t hfx_preprocess(hfx_ctx *ctx, const hfx_search_params *p, const float *mz
     if (e) return cuda_fail(ctx, e, "alloc");
     uint32_t *d_max = ctx->buf<uint32_t>("maxlen", 4, e);
     if (e) return cuda_fail(ctx, e, "alloc");
-    float *tol = ctx->buf<float>("tol0", nspec, e);
-    if (e) return cuda_fail(ctx, e, "alloc");
-    HFX_CUDA(cudaMemsetAsync(tol, 0, 4ull * nspec, ctx->stream), "memset");
-    int rc = hfx_launch_layout(mz, off, pcr, z, tol, nspec, lp, meta, d_max, nullptr, ctx->stream);
+    int rc = hfx_launch_layout(mz, off, pcr, z, nullptr, nspec, lp, meta, d_max, nullptr, ctx->stream, lens, masses);
     if (rc) return cuda_fail(ctx, (cudaError_t)rc, "k_layout");
     HFX_CUDA(ctx->d_err.ensure(16), "alloc err");
     HFX_CUDA(clear_err(ctx), "memset err");
     rc = hfx_launch_preprocess(mz, it, off, pcr, lp, meta, nspec, stride, rows, (__nv_bfloat16 *)rows_bf16,
                                (__half *)rows_fp16, ctx->d_err.as<uint32_t>(), ctx->stream);
     if (rc) return cuda_fail(ctx, (cudaError_t)rc, "k_preprocess");
-    std::vector<SpecMeta> hm(nspec);
-    HFX_CUDA(cudaMemcpyAsync(hm.data(), meta, sizeof(SpecMeta) * nspec, cudaMemcpyDeviceToHost, ctx->stream), "D2H");
     HFX_CUDA(cudaStreamSynchronize(ctx->stream), "sync");
-    std::vector<int32_t> hl(nspec);
-    std::vector<float> hmass(nspec);
-    for (int32_t s = 0; s < nspec; ++s) {
-        hl[s] = hm[s].status == 0 ? hm[s].len : 0;
-        hmass[s] = hm[s].mass;
-    }
-    if (lens) HFX_CUDA(cudaMemcpy(lens, hl.data(), 4ull * nspec, cudaMemcpyHostToDevice), "H2D lens");
-    if (masses) HFX_CUDA(cudaMemcpy(masses, hmass.data(), 4ull * nspec, cudaMemcpyHostToDevice), "H2D masses");
     return HFX_OK;
 }
 
