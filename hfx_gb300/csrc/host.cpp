@@ -595,7 +595,7 @@ int32_t search_batched(hfx_ctx *ctx, const hfx_search_params *p, const Batch &b,
     // one 16-byte tile load per bin: 8 BF16/FP16 or 4 FP32 spectra per group;
     // half of that over isoform lists, whose windows few spectra share (1.5 of
     // 8 on average with 2,000 spectra): two of the smaller tiles fit an SM, and
-    // the scorer took 15.0 against 22.2 ms (FP32, 1,000 spectra: 2.6 against 3.5)
+    // the scorer took 14.0 against 22 ms (FP32, 1,000 spectra: 2.6 against 3.5)
     const bool iso = p->batch_mode == 1 && p->search_mods != 0 && ctx->num_mod > 0;
     int32_t G = p->group_size > 0 ? p->group_size : (elem_kind == 0 ? 4 : 8) / (iso ? 2 : 1);
     const int32_t chunk = p->chunk > 0 ? p->chunk : 4096;

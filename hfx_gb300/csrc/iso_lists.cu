@@ -317,45 +317,6 @@ __global__ void __launch_bounds__(256, kClass == 0 ? 1 : 4) k_gen_iso_lists(DevD
     }
 }
 
-// A lane's entries of one round over a list of n.  EntryRound: entry k of the
-// round's 4 W is lane k % W's, the canonical order of FP32 sums.
-template <int W>
-struct EntryRound {
-    static constexpr int kPer = 4, kRound = 4 * W;
-    uint32_t e[4];
-    __device__ __forceinline__ void load(const uint16_t *lp, int i0, int hl, int n, uint32_t pad) {
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const int i = i0 + W * k + hl;
-            e[k] = i < n ? (uint32_t)__ldg(lp + i) : pad;
-        }
-    }
-    __device__ __forceinline__ uint32_t at(int k) const { return e[k]; }
-};
-// EntryVector: eight neighbouring entries a lane in one 16-byte load (lists start
-// on 16-byte boundaries and own the rest of their last one).  BF16/FP16 sums only
-// choose what FP32 rescoring orders.
-template <int W>
-struct EntryVector {
-    static constexpr int kPer = 8, kRound = 8 * W;
-    uint32_t v[4];
-    __device__ __forceinline__ void load(const uint16_t *lp, int i0, int hl, int n, uint32_t pad) {
-        const int i = i0 + 8 * hl;
-        uint4 u = make_uint4(0u, 0u, 0u, 0u);
-        if (i < n) u = __ldg(reinterpret_cast<const uint4 *>(lp + i));
-        v[0] = u.x, v[1] = u.y, v[2] = u.z, v[3] = u.w;
-        if (i + 8 > n) {
-            // past the list's end
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                if (i + 2 * k >= n) v[k] = pad | pad << 16;
-                else if (i + 2 * k + 1 >= n) v[k] = (v[k] & 0xFFFFu) | pad << 16;
-            }
-        }
-    }
-    __device__ __forceinline__ uint32_t at(int k) const { return k & 1 ? v[k >> 1] >> 16 : v[k >> 1] & 0xFFFFu; }
-};
-
 // 5. the scorer over the isoform lists: a persistent grid pulls work items
 // (group, combination, chunk of positions); the group's tile is staged by
 // one bulk copy; an item's isoforms are [index(mu, p0), index(mu, p1)); kC
@@ -363,10 +324,10 @@ struct EntryVector {
 // partial-sum sets, the canonical order.  One isoform meets 1.5 spectra of a
 // group, so what it costs beside the FMAs decides: loads that waited for one
 // another (the key, the offset, each round of entries), and the admission of
-// four scores by turns where none is admitted.  In a pipeline, with 16-byte list
-// loads, the admission only where a score beats a list's last, and two CTAs an
-// SM (tiles of 8 bytes a bin), the 16 M isoforms of 2,000 spectra against 20,000
-// proteins took 15.0 ms instead of 22.2; bound by instructions issued (67 %).
+// four scores by turns where none is admitted.  In a pipeline, with the
+// admission only where a score beats a list's last, and two CTAs an SM (tiles of
+// 8 bytes a bin), the 16 M isoforms of 2,000 spectra against 20,000 proteins
+// took 14.0 ms instead of 22.2; bound by instructions issued (67 %).
 template <typename T, int G, int kC>
 __global__ void __launch_bounds__(512, G * sizeof(T) <= 8 ? 2 : 1)
 k_score_iso_lists(const uint16_t *__restrict__ lists, uint64_t list_total, const uint32_t *__restrict__ lstart,
@@ -387,7 +348,7 @@ k_score_iso_lists(const uint16_t *__restrict__ lists, uint64_t list_total, const
     // this lane's partial set k (8 lanes per isoform)
     constexpr bool kSets4 = std::is_same<T, float>::value && kC > 1;
     static_assert(G <= kW, "a lane group takes up to one spectrum of the group per lane");
-    using Entries = typename std::conditional<kSets4, EntryRound<kW>, EntryVector<kW>>::type;
+    using Entries = EntryRound<uint16_t, kW>;
     extern __shared__ __align__(128) uint8_t smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int hl = lane & (kW - 1), quad = lane / kW;
@@ -568,14 +529,13 @@ k_score_iso_lists(const uint16_t *__restrict__ lists, uint64_t list_total, const
             // the round's entries, the next round's already in flight
             Entries e = cur.e;
             for (int i0 = 0; i0 < nmax; i0 += Entries::kRound) {
-                Entries f = e;
-                if (kSets4 || i0 + Entries::kRound < nmax) f.load(cur.lp, i0 + Entries::kRound, hl, n, pad);
+                Entries f;
+                f.load(cur.lp, i0 + Entries::kRound, hl, n, pad);
 #pragma unroll
-                for (int k = 0; k < Entries::kPer; ++k) {
+                for (int k = 0; k < 4; ++k) {
                     float *a = acc;
-                    if constexpr (kSets4) a = acc4[k & 3];
-                    const uint32_t w = e.at(k);
-                    TileFma<T, G>::fma(stile, w >> 2, w & 3u, *reinterpret_cast<float(*)[G]>(a));
+                    if constexpr (kSets4) a = acc4[k];
+                    TileFma<T, G>::fma(stile, e.e[k] >> 2, e.e[k] & 3u, *reinterpret_cast<float(*)[G]>(a));
                 }
                 e = f;
             }

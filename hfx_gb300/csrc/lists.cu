@@ -431,6 +431,7 @@ k_score_lists(const E *__restrict__ lists, const uint32_t *__restrict__ lstart, 
     constexpr bool kSets4 = std::is_same<T, float>::value && kC > 1;
     static_assert(!kSets4 || kW == 8, "the FP32 partial-sum sets assume 8 lanes per candidate");
     static_assert(G <= kW, "a lane group takes up to one spectrum of the group per lane");
+    using Entries = EntryRound<E, kW>;
     extern __shared__ __align__(128) uint8_t smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int hl = lane & (kW - 1), half = lane / kW;  // `half`: the lane's candidate group
@@ -536,7 +537,7 @@ k_score_lists(const E *__restrict__ lists, const uint32_t *__restrict__ lstart, 
             int n;
             bool live;
             const E *lp;
-            uint32_t e[4];
+            Entries e;
         };
         auto claim = [&]() {
             Meta m;
@@ -577,11 +578,7 @@ k_score_lists(const E *__restrict__ lists, const uint32_t *__restrict__ lstart, 
                     c.lp = lists + off;
                 }
             }
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const int i = kW * k + hl;
-                c.e[k] = i < c.n ? (uint32_t)__ldg(c.lp + i) : pad;
-            }
+            c.e.load(c.lp, 0, hl, c.n, pad);
             return c;
         };
         Meta ahead = claim();
@@ -609,36 +606,27 @@ k_score_lists(const E *__restrict__ lists, const uint32_t *__restrict__ lstart, 
 #pragma unroll
             for (int o = kW; o < 32; o <<= 1) nmax = max(nmax, __shfl_xor_sync(kFullMask, nmax, o));
             // entries [i0, i0 + 4 kW) in e, the next 4 kW already in flight in f
-            uint32_t e[4], f[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                e[k] = cur.e[k];
-                const int i = 4 * kW + kW * k + hl;
-                f[k] = i < n ? (uint32_t)__ldg(cur.lp + i) : pad;
-            }
+            Entries e = cur.e, f;
+            f.load(cur.lp, 4 * kW, hl, n, pad);
             for (int i0 = 0; i0 < nmax; i0 += 4 * kW) {
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
-                    const uint32_t bin = e[k] >> 2;
+                    const uint32_t w = e.e[k], bin = w >> 2;
                     float *a = acc;
                     if constexpr (kSets4) a = acc4[k];
                     if constexpr (kGlobal) {
                         if ((int32_t)bin < nb)
-                            TileFma<T, G>::fma(tile, bin, e[k] & 3u, *reinterpret_cast<float(*)[G]>(a));
+                            TileFma<T, G>::fma(tile, bin, w & 3u, *reinterpret_cast<float(*)[G]>(a));
                     } else {
                         // zero beyond nb
-                        TileFma<T, G>::fma(tile, bin, e[k] & 3u, *reinterpret_cast<float(*)[G]>(a));
+                        TileFma<T, G>::fma(tile, bin, w & 3u, *reinterpret_cast<float(*)[G]>(a));
                     }
                 }
                 // lists ascend: once an entry lies beyond the tile, so do the rest
-                const uint32_t last = __shfl_sync(kFullMask, e[3], (lane & ~(kW - 1)) | (kW - 1));
+                const uint32_t last = __shfl_sync(kFullMask, e.e[3], (lane & ~(kW - 1)) | (kW - 1));
                 if (__all_sync(kFullMask, (last >> 2) >= (uint32_t)nb)) break;
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    e[k] = f[k];
-                    const int i = i0 + 8 * kW + kW * k + hl;
-                    f[k] = i < n ? (uint32_t)__ldg(cur.lp + i) : pad;
-                }
+                e = f;
+                f.load(cur.lp, i0 + 8 * kW, hl, n, pad);
             }
             if constexpr (kSets4) {
                 // offsets 16 (partials l and l + 16, l + 8 and l + 24) and 8
@@ -648,32 +636,38 @@ k_score_lists(const E *__restrict__ lists, const uint32_t *__restrict__ lstart, 
             }
             if constexpr (kC > 1) {
                 const float sc = reduce_scatter_lanes<G, kW>(acc);
+                if (hl == 0 && cur.act) {
+                    my_cand += 1u;
+                    my_entries += (uint32_t)n;
+                    my_psm += (uint32_t)__popc(cur.act);
+                }
+                // lane j * kW / G of a candidate's lanes has member j's score
+                const int mine = hl / (kW / G);
+                const bool holds = (hl & (kW / G - 1)) == 0 && ((cur.act >> mine) & 1u);
+                // every pair's score, at its member's window offset
+                // (E-values; FP32 only, the host refuses a sink otherwise)
+                if constexpr (std::is_same<T, float>::value) {
+                    if (sink && holds) sink[s_off[mine] + (cur.p - s_wb[mine])] = sc;
+                }
+                // the queues take the four when one beats its list's last
+                if (!__any_sync(kFullMask, holds && score_order(sc) >= *(volatile uint32_t *)(thr_u + mine))) continue;
                 const bool owner = (lane & (32 / G - 1)) == 0;
 #pragma unroll
                 for (int q = 0; q < kC; ++q) {
                     const uint32_t act_q = __shfl_sync(kFullMask, cur.act, q * kW);
                     const uint32_t p_q = __shfl_sync(kFullMask, cur.p, q * kW);
-                    const int n_q = __shfl_sync(kFullMask, n, q * kW);
-                    my_cand += act_q != 0u;
-                    my_entries += (uint32_t)n_q;
-                    my_psm += (uint32_t)__popc(act_q);
-                    // member j's sums sit in lanes j * kW / G of candidate q's
-                    // group; its admission lane is j * 32 / G
+                    // member j's admission lane is j * 32 / G
                     const float sc_q = __shfl_sync(kFullMask, sc, q * kW + (lane / (32 / G)) * (kW / G));
-                    // every pair's score, at its member's window offset
-                    // (E-values; FP32 only, the host refuses a sink otherwise)
-                    if constexpr (std::is_same<T, float>::value) {
-                        if (sink && owner && ((act_q >> my_slot) & 1u))
-                            sink[s_off[my_slot] + (p_q - s_wb[my_slot])] = sc_q;
-                    }
                     const bool want = owner && ((act_q >> my_slot) & 1u) &&
                                       score_order(sc_q) >= *(volatile uint32_t *)(thr_u + my_slot);
                     slots.offer(want, sc_q, p_q, my_slot, K);
                 }
             } else {
-                my_cand += 1u;
-                my_entries += (uint32_t)n;
-                my_psm += (uint32_t)__popc(cur.act);
+                if (lane == 0) {
+                    my_cand += 1u;
+                    my_entries += (uint32_t)n;
+                    my_psm += (uint32_t)__popc(cur.act);
+                }
                 const float sc = reduce_scatter<G>(acc);
                 if (sink) {
                     // every pair's score, at its member's window offset (the
@@ -695,7 +689,7 @@ k_score_lists(const E *__restrict__ lists, const uint32_t *__restrict__ lstart, 
         __syncthreads();
     }
     if (stats) {
-        if (lane == 0) {
+        if (hl == 0) {
             atomicAdd(&s_stats[0], (unsigned long long)my_cand);
             atomicAdd(&s_stats[1], (unsigned long long)my_entries);
             atomicAdd(&s_stats[2], (unsigned long long)my_psm);
