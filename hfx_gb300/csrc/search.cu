@@ -8,37 +8,33 @@ namespace hfx {
 
 // Stage (b), filter.cu:75-127: begin = lower_bound(r_sorted, m - eps),
 // end = upper_bound(r_sorted, m + eps), both bounds inclusive.
-__device__ __forceinline__ uint32_t lower_bound_f(const float *a, uint32_t n, float v) {
-    uint32_t lo = 0, hi = n;
-    while (lo < hi) {
-        uint32_t mid = (lo + hi) >> 1;
-        if (a[mid] < v) lo = mid + 1; else hi = mid;
-    }
-    return lo;
-}
-__device__ __forceinline__ uint32_t upper_bound_f(const float *a, uint32_t n, float v) {
-    uint32_t lo = 0, hi = n;
-    while (lo < hi) {
-        uint32_t mid = (lo + hi) >> 1;
-        if (v < a[mid]) hi = mid; else lo = mid + 1;
-    }
-    return lo;
-}
-
-// Two threads per spectrum: the even one searches the lower bound, the odd
-// one the upper, so the two chains of dependent loads run at once.
-__global__ void k_windows(const float *__restrict__ r_sorted, uint32_t n, const SpecMeta *__restrict__ meta,
-                          int32_t nspec, uint32_t *__restrict__ wb, uint32_t *__restrict__ we) {
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int32_t s = (int32_t)(t >> 1);
-    const bool upper = t & 1;
-    uint32_t x = 0;
-    if (s < nspec && meta[s].status == 0)
-        x = upper ? upper_bound_f(r_sorted, n, meta[s].hi) : lower_bound_f(r_sorted, n, meta[s].lo);
-    const uint32_t b = __shfl_sync(kFullMask, x, (threadIdx.x & 31) & ~1);
+// A warp per spectrum: lanes 0-15 search the lower bound, 16-31 the upper.  The
+// search is one chain of dependent loads, so each round asks for 16 places at
+// once: 5 rounds over 1.3 M masses instead of 20 (14 us of a one-spectrum search
+// with a thread per bound).
+__global__ void __launch_bounds__(128) k_windows(const float *__restrict__ r_sorted, uint32_t n,
+                                                 const SpecMeta *__restrict__ meta, int32_t nspec,
+                                                 uint32_t *__restrict__ wb, uint32_t *__restrict__ we) {
+    const int lane = threadIdx.x & 31, l = lane & 15;
+    const int32_t s = (int32_t)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     if (s >= nspec) return;
-    if (upper) we[s] = x < b ? b : x;
-    else wb[s] = x;
+    const bool upper = lane >= 16;
+    uint32_t lo = 0, hi = meta[s].status == 0 ? n : 0u;
+    const float v = upper ? meta[s].hi : meta[s].lo;
+    while (__any_sync(kFullMask, lo < hi)) {
+        const uint32_t step = (hi - lo) / 17u + 1u, at = lo + (uint32_t)(l + 1) * step - 1u;
+        bool before = false;  // the bound lies past `at`
+        if (at < hi) {
+            const float r = __ldg(r_sorted + at);
+            before = upper ? !(v < r) : r < v;
+        }
+        const uint32_t c = (uint32_t)__popc((__ballot_sync(kFullMask, before) >> (lane & 16)) & 0xFFFFu);
+        if (c < 16u) hi = min(hi, lo + (c + 1u) * step - 1u);
+        lo += c * step;
+    }
+    const uint32_t b = __shfl_sync(kFullMask, lo, 0);
+    if (lane == 0) wb[s] = lo;
+    if (lane == 16) we[s] = lo < b ? b : lo;
 }
 
 // Write every warp's list to shared memory and merge them in warp 0.
@@ -217,7 +213,7 @@ static size_t score_smem_bytes(int32_t len, int32_t words, int nw, int K) {
 int hfx_launch_windows(const float *r_sorted, uint32_t n, const SpecMeta *meta, int32_t nspec, uint32_t *wb,
                        uint32_t *we, cudaStream_t st) {
     if (nspec <= 0) return 0;
-    k_windows<<<(unsigned)((2ll * nspec + 127) / 128), 128, 0, st>>>(r_sorted, n, meta, nspec, wb, we);
+    k_windows<<<(unsigned)((nspec + 3ll) / 4), 128, 0, st>>>(r_sorted, n, meta, nspec, wb, we);
     return (int)cudaGetLastError();
 }
 
