@@ -79,3 +79,33 @@ def test_rows_at_their_edges(gpulib, oracle, stride, infinite):
         assert torch.equal(rbf[i][keep], rows[i][keep].bfloat16())
         assert torch.equal(rh[i][keep], rows[i][keep].half())
     eng.close()
+
+
+@pytest.mark.parametrize("npk", [1, 2, 511, 512, 513, 1100])
+def test_sparse_rows_by_peaks(gpulib, oracle, npk):
+    """0.02 Da rows: the forms for up to 512 peaks and for more, peaks alone, in
+    crowds (many to a window) and at the row's ends."""
+    torch = pytest.importorskip("torch")
+    import hfx_gb300
+    rng = np.random.default_rng(npk)
+    mz = np.sort(np.concatenate([rng.uniform(0.0, 1400.0, npk - npk // 2 - 1), rng.uniform(700.0, 706.0, npk // 2),
+                                 [1400.0]]))[:npk].astype(np.float32)
+    it = rng.lognormal(0.0, 2.0, size=npk).astype(np.float32)
+    pcr, z = np.array([900.0], np.float32), np.array([2.0], np.float32)
+    x = oracle.preprocess(mz, it, pcr[0], z[0], bw=0.02, custom_bw=True, remove_pcr=False)
+    stride = 16 * ((len(x) + 15) // 16 if x is not None else 1)
+    stride = max(stride, 16 * 4000)
+    dev = dict(mz=mz, it=it, off=np.array([0, npk], np.int64), pcr=pcr, z=z)
+    dev = {k: torch.from_numpy(v).cuda() for k, v in dev.items()}
+    eng = hfx_gb300.Engine(0)
+    rows = torch.full((1, stride), 7.0, device="cuda")
+    rbf = torch.full((1, stride), 7.0, dtype=torch.bfloat16, device="cuda")
+    eng.preprocess(dev, hfx_gb300.default_params(bin_width=0.02, custom_bin_width=1, remove_precursor_peak=0), stride,
+                   rows, rbf)
+    torch.cuda.synchronize()
+    want = np.zeros(stride, np.float32)
+    if x is not None:
+        want[:len(x)] = x
+    assert np.array_equal(rows[0].cpu().numpy().view(np.uint32), want.view(np.uint32))
+    assert torch.equal(rbf[0], rows[0].bfloat16())
+    eng.close()
