@@ -10,8 +10,8 @@ search's).  `value` times steps whose inputs are already resident in HBM
 with pinned host buffers, copies included.  Between timed steps the L2 is
 flushed by writing a 512 MB buffer (outside the timed events).
 
-Beside the headline the line carries the plain FP32 path (one launch per
-spectrum) timed on the same spectra and its top-10 agreement; `parity`: the
+Beside the headline the line carries the plain FP32 path (every spectrum by
+its own blocks) timed on the same spectra and its top-10 agreement; `parity`: the
 timed search's top-10 keys, FP32 scores and candidate counts compared bit
 for bit with the oracle's FP32 search of every spectrum (the +-3 Da
 workloads; a sample of the open-window ones) and its agreement with the
@@ -62,22 +62,22 @@ KERNEL_SRC = {
     "k_score_iso_lists": ["hfx_gb300/csrc/iso_lists.cu", "hfx_gb300/csrc/mods_device.cuh"] + _COMMON_SRC,
 }
 # Scaled captures: the DRAM bytes (and the warp instructions, `inst`) of one
-# launch on the 2,000-spectrum (full) or 1,000-spectrum (mods) case, times
-# the ratio of the full-size launch's moved bytes (the run's work counters,
+# launch (the generators: of their four) on the 2,000-spectrum (full) or
+# 500-spectrum (mods) case, times the ratio of the full-size launch's moved bytes (the run's work counters,
 # per-kernel basis below) to the small case's.
 TRAFFIC = {
     ("k_gen_lists", "full", 1, 10000): {
-        "src": "514a0af75598", "bytes": 2205793354, "inst": 4522799000,
+        "src": "2c86f8c5f15c", "bytes": 1969009253, "inst": 1909988937,
         "profile": "profiles/k_gen_lists_2k_bf16.md (2,000-spectrum capture x 1.729 moved-bytes ratio)"},
     ("k_score_lists", "full", 1, 10000): {
-        "src": "514a0af75598", "bytes": 3319129096, "inst": 2310847000,
+        "src": "2c86f8c5f15c", "bytes": 3320183081, "inst": 2170058895,
         "profile": "profiles/k_score_lists_2k_bf16.md (2,000-spectrum capture x 2.482 moved-bytes ratio)"},
     ("k_gen_iso_lists", "mods", 1, 10000): {
-        "src": "b9b44833cf01", "bytes": 50181657886, "inst": 91095407000,
-        "profile": "profiles/iso_lists_mods1k_bf16.md (1,000-spectrum capture x 3.904 moved-bytes ratio)"},
+        "src": "606c66706d60", "bytes": 50460321735, "inst": 56449742430,
+        "profile": "profiles/iso_lists_mods_bf16.md (500-spectrum capture x 6.986 moved-bytes ratio)"},
     ("k_score_iso_lists", "mods", 1, 10000): {
-        "src": "b9b44833cf01", "bytes": 62823028595, "inst": 31125280000,
-        "profile": "profiles/iso_lists_mods1k_bf16.md (1,000-spectrum capture x 4.815 moved-bytes ratio)"},
+        "src": "606c66706d60", "bytes": 74375970086, "inst": 38759597972,
+        "profile": "profiles/iso_lists_mods_bf16.md (500-spectrum capture x 10.258 moved-bytes ratio)"},
 }
 
 
