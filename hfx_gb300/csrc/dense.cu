@@ -72,8 +72,7 @@ __host__ __device__ __forceinline__ uint32_t swizzled(uint32_t r, uint32_t k) {
 // 0.64 ns whatever the block's windows (18 M rows in 10.5 ms), a pair of the list
 // scorer 0.038 ns.  With the line at 16 the +-3 Da blocks of 10,000 spectra that
 // passed it made their scoring slower (2.78 -> 3.15 ms); at 32 none of them does,
-// and open windows have 36 to 115.
-constexpr uint32_t kDenseMinPairs = 32;
+// and open windows have 36 to 115 (kDenseMinPairs).
 constexpr uint32_t kDenseMinWidth = 4096;
 
 // One warp per block.  Classes as in k_groups.

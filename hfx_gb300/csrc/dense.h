@@ -5,6 +5,8 @@
 
 namespace hfx {
 
+// A block is one from this many pairs per candidate of its union on (dense.cu).
+constexpr int32_t kDenseMinPairs = 32;
 constexpr int kDenseSpectra = 128;  // spectra per block: the rows of one MMA
 constexpr int kDenseQueue = 16;     // queued candidates per spectrum
 

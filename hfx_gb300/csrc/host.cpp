@@ -636,8 +636,10 @@ int32_t search_batched(hfx_ctx *ctx, const hfx_search_params *p, const Batch &b,
     if (e) return cuda_fail(ctx, e, "alloc");
     // wide windows on the tensor cores: unmodified candidates, lists, up to 32
     // kept, and without a score sink; an FP32 search keeps 32 then and rescores
-    // them, so it has to ask for few enough of them
-    const bool dense_on = lists_only && !long_rows && K <= 32 && p->search_plain != 0 &&
+    // them, so it has to ask for few enough of them.  A block's pairs are at most
+    // its spectra times their union, so fewer spectra than the rule's share have
+    // no block and need no plan of them (15 us of a one-spectrum search)
+    const bool dense_on = lists_only && !long_rows && K <= 32 && p->search_plain != 0 && ns >= kDenseMinPairs &&
                           (elem_kind != 0 || (p->top_n <= 16 && !ctx->ev_single));
     DenseWs dw{};
     if (dense_on) {
