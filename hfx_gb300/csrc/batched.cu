@@ -112,6 +112,45 @@ __global__ void k_bucket_scatter(const SpecMeta *__restrict__ meta, int32_t nspe
     perm[pos] = s;
 }
 
+// The same for up to kSortFew spectra, by one block without the buckets: a
+// spectrum's place is the number of smaller keys (bucket, then number), counted
+// over the keys in shared memory.  Of the buckets' ends only the classes' are
+// read.  A one-spectrum search took 26 us to clear, count, scan and fill the
+// 98,304 buckets; this takes 3 us, and 8 us for 517 spectra, 18 us for 1,024.
+__global__ void __launch_bounds__(kSortFew) k_sort_few(const SpecMeta *__restrict__ meta, int32_t nspec,
+                                                       uint32_t *__restrict__ bucket_end,
+                                                       uint32_t *__restrict__ n_sorted, int32_t *__restrict__ perm) {
+    __shared__ __align__(16) uint32_t keys[kSortFew];
+    __shared__ uint32_t in_class[kClasses];
+    const int t = threadIdx.x;
+    uint32_t key = ~0u;  // no row, or no spectrum
+    if (t < kClasses) in_class[t] = 0u;
+    __syncthreads();
+    if (t < nspec) {
+        const SpecMeta m = meta[t];
+        if (m.status == 0) {
+            key = (uint32_t)spec_bucket(m) << 10 | (uint32_t)t;
+            atomicAdd(&in_class[spec_class(m)], 1u);
+        }
+    }
+    keys[t] = key;
+    __syncthreads();
+    if (key != ~0u) {
+        uint32_t at = 0;
+        for (int j = 0; j < nspec; j += 4) {
+            const uint4 k = *reinterpret_cast<const uint4 *>(keys + j);
+            at += (k.x < key) + (k.y < key) + (k.z < key) + (k.w < key);
+        }
+        perm[at] = t;
+    }
+    if (t < kClasses) {
+        uint32_t end = 0;
+        for (int c = 0; c <= t; ++c) end += in_class[c];
+        bucket_end[(t + 1) * kMassBuckets - 1] = end;
+        if (t == kClasses - 1) *n_sorted = end;
+    }
+}
+
 // With few_groups (no work-item size asked for) a group's window is cut so
 // that about this many items come of all groups together, four per resident
 // CTA of the list scorer: one spectrum's 3,400 candidates in one item kept one
@@ -499,11 +538,15 @@ size_t hfx_batched_smem(int64_t stride, int elem_bytes, int G, int nw, int K) {
 int hfx_batched_plan(const SpecMeta *meta, int32_t nspec, const uint32_t *wb, const uint32_t *we, int32_t G,
                      int32_t chunk, int few_groups, const BatchedWs &ws, const DenseWs *dw, cudaStream_t st) {
     const int nbk = kClasses * kMassBuckets;
-    cudaMemsetAsync(ws.hist, 0, sizeof(uint32_t) * (nbk + 1), st);
     cudaMemsetAsync(ws.item_off, 0, sizeof(uint32_t) * (nspec + 1), st);
-    k_bucket_count<<<(nspec + 255) / 256, 256, 0, st>>>(meta, nspec, ws.hist);
-    k_scan_u32<<<1, 1024, 0, st>>>(ws.hist, nbk, ws.n_sorted);
-    k_bucket_scatter<<<(nspec + 255) / 256, 256, 0, st>>>(meta, nspec, ws.hist, ws.perm);
+    if (nspec <= kSortFew) {
+        k_sort_few<<<1, kSortFew, 0, st>>>(meta, nspec, ws.hist, ws.n_sorted, ws.perm);
+    } else {
+        cudaMemsetAsync(ws.hist, 0, sizeof(uint32_t) * (nbk + 1), st);
+        k_bucket_count<<<(nspec + 255) / 256, 256, 0, st>>>(meta, nspec, ws.hist);
+        k_scan_u32<<<1, 1024, 0, st>>>(ws.hist, nbk, ws.n_sorted);
+        k_bucket_scatter<<<(nspec + 255) / 256, 256, 0, st>>>(meta, nspec, ws.hist, ws.perm);
+    }
     const int32_t max_groups = nspec;  // each class adds at most one partial group
     k_groups<<<(max_groups + 255) / 256, 256, 0, st>>>(ws.hist, ws.n_sorted, ws.perm, wb, we, meta, G, chunk,
                                                        few_groups, max_groups, ws.groups, ws.item_off, ws.group_of, ws.slot_of,

@@ -27,6 +27,7 @@ struct BatchedWs {
 };
 
 constexpr int kBucketCount = 12 * 8192;
+constexpr int kSortFew = 1024;      // spectra that one block sorts without the buckets
 struct DenseWs;
 }  // namespace hfx
 

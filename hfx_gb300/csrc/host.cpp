@@ -675,7 +675,8 @@ int32_t search_batched(hfx_ctx *ctx, const hfx_search_params *p, const Batch &b,
     rc = hfx_batched_plan(meta, ns, wb, we, G, chunk, p->chunk > 0 ? 0 : 1, ws, dense_on ? &dw : nullptr,
                           ctx->stream);
     if (rc) return cuda_fail(ctx, (cudaError_t)rc, "plan");
-    ctx->stage_end(HFX_STAGE_WINDOWS, dense_on ? 8 : 6, ns);  // k_windows + the planning kernels
+    // k_windows + the planning kernels
+    ctx->stage_end(HFX_STAGE_WINDOWS, (dense_on ? 8 : 6) - (ns <= kSortFew ? 2 : 0), ns);
     uint32_t ngroups = 0, total_items = 0, ntiles = 0, ditems = 0;
     if (ctx->gmode >= 1) {
         // capacities of the graph; a batch that needs more is reported (k_clamp_items)
