@@ -21,8 +21,14 @@
 // and 8e-6 (1e-6 with six) of smaller ones; over values spread evenly in their
 // exponents the RMS error is 0.76 of BF16's and 0.14 of FP16's, and six pieces
 // move a score by about 1e-8 of itself (FP32 summation: 6e-8).  The scores only
-// choose the candidates that FP32 rescoring orders in the canonical order; FP32
-// searches keep 32 of them for at most 16 results.
+// choose the candidates that FP32 rescoring orders in the canonical order.
+//
+// FP32 searches keep 32 candidates for at most 16 results, and the results have
+// to be those of scoring every pair in FP32: after the rescoring k_dense_prove
+// bounds how far a score of the pieces can be from the FP32 score, and a spectrum
+// whose last result is not above the 32nd kept score by more than that (spectra of
+// a few peaks, where hundreds of candidates tie) is scored again by the list
+// scorer.
 //
 // Work.  An item is 128 spectra times a run of candidates, taken 512 at a time
 // (512 columns of 128 FP32 accumulators fill the SM's tensor memory).  For each
@@ -150,6 +156,7 @@ __global__ void k_dense_plan(const SpecMeta *__restrict__ meta, const uint32_t *
         const uint32_t even = 136u / (((uint32_t)maxlen + 127u) / 128u);
         d.chunk = max((uint32_t)min(share, (unsigned long long)even), 1u) * kDenseRows;
         d.tile = atomicAdd(dw.n_tiles, 1u);
+        d.ladder = 0u;
         dw.blocks[b] = d;
         dw.tile_block[d.tile] = (uint32_t)b;
         dw.item_off[b] = (hi - lo + d.chunk - 1) / d.chunk;
@@ -677,6 +684,100 @@ k_dense_score(const uint16_t *__restrict__ lists, uint64_t list_total, const uin
     }
 }
 
+// ---- FP32 searches: are the results certain? ----
+//
+// A candidate that was not kept has a score of the pieces p of at most p32, the
+// 32nd kept one's, and its FP32 score is at most p + E.  With a list of n entries
+// and total weight T, N the sum of weight x |x| over the list's negative values and
+// M = p32 + N (no partial sum of either is larger):
+//   products and accumulators: at most 6 n products that are not zero and one
+//     accumulator per MMA, each off by no more than 2^-22 M -- twice the unit of an
+//     FP32 sum that truncates (measured: 1.5e-7 of a score, some 10^-4 of E),
+//   row values: T 2^-20 (six pieces),
+//   the canonical FP32 sum: (n / 32 + 6) 2^-24 (M + N).
+// n and T come of the block's longest ladder, L prefixes: 10 L z entries (or all
+// bins) and weights 240 L z; N is at most T times the row's lowest value and 50
+// times the sum of its negative ones.  Of spectra
+// with 50 to 400 peaks (20,000 proteins, +-500 Da) the tenth result lies 570 to
+// 2,900 above the 32nd, E is 10 to 200.  The rescored candidates are checked
+// against E themselves.  A warp per spectrum, bound by reading its row once.
+__global__ void __launch_bounds__(256) k_dense_ladders(const uint32_t *__restrict__ tc, const uint32_t *__restrict__ tn,
+                                                       DenseWs dw) {
+    const uint32_t b = blockIdx.x;
+    if (dw.item_off[b] == dw.item_off[b + 1]) return;  // not dense
+    const uint32_t hi = dw.blocks[b].hi;
+    uint32_t ladder = 0;
+    for (uint32_t p = dw.blocks[b].lo + blockIdx.y * blockDim.x + threadIdx.x; p < hi; p += gridDim.y * blockDim.x)
+        ladder = max(ladder, tn[p] > tc[p] ? tn[p] - tc[p] : 0u);
+    ladder = __reduce_max_sync(kFullMask, ladder);
+    if ((threadIdx.x & 31) == 0) atomicMax(&dw.blocks[b].ladder, ladder);
+}
+
+__global__ void __launch_bounds__(128) k_dense_prove(
+    const SpecMeta *__restrict__ meta, const int32_t *__restrict__ group_of, const GroupInfo *__restrict__ groups,
+    const DenseBlock *__restrict__ blocks, const uint32_t *__restrict__ wb, const uint32_t *__restrict__ we,
+    const float *__restrict__ rows, int64_t stride, const float *__restrict__ kept_s, const uint64_t *__restrict__ kept_k, int32_t nspec,
+    int32_t topn, const float *__restrict__ out_s, const uint64_t *__restrict__ out_k,
+    SpecMeta *__restrict__ open_meta, uint32_t *__restrict__ n_open) {
+    constexpr int kKept = 32;
+    const int lane = threadIdx.x & 31;
+    const int32_t s = (int32_t)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    if (s >= nspec) return;
+    SpecMeta m = meta[s];
+    int32_t b = -1;
+    if (m.status == 0) b = groups[group_of[s]].block;
+    bool certain = true;  // no row, list-scored, or every candidate kept
+    if (b >= 0 && we[s] - wb[s] > (uint32_t)kKept) {
+        const DenseBlock d = blocks[b];
+        float low = 0.0f;
+        double neg = 0.0;
+        for (int32_t i = lane; i < m.len; i += 32) {
+            const float x = fminf(rows[(size_t)s * stride + i], 0.0f);
+            low = fminf(low, x);
+            neg -= (double)x;
+        }
+        for (int o = 16; o >= 1; o >>= 1) {
+            low = fminf(low, __shfl_xor_sync(kFullMask, low, o));
+            neg += __shfl_xor_sync(kFullMask, neg, o);
+        }
+        const double ions = (double)d.ladder * (double)m.charges_plain, weight = 240.0 * ions;
+        const double n = fmin(10.0 * ions, (double)m.len);
+        const double to_score = 5.0 / (double)kDenseScale;
+        const double p32 = to_score * (double)kept_s[(size_t)s * kKept + kKept - 1];
+        const double N = fmin(weight * -(double)low, 50.0 * neg), M = fmax(p32, 0.0) + N;
+        const double mmas = 6.0 * 4.0 * (double)((d.maxlen + 127) / 128);
+        const double E = 1.01 * ((6.0 * n + mmas) * 0x1p-22 * M + weight * 0x1p-20 +
+                                 (n / 32.0 + 6.0) * 0x1p-24 * (M + N));
+        certain = (double)out_s[(size_t)s * topn + topn - 1] > p32 + E;
+        if (lane < topn) {  // each result's own two scores
+            const uint64_t k = out_k[(size_t)s * topn + lane];
+            const double f = (double)out_s[(size_t)s * topn + lane];
+            bool near = false;
+            for (int t = 0; t < kKept; ++t)
+                if (kept_k[(size_t)s * kKept + t] == k)
+                    near = fabs(to_score * (double)kept_s[(size_t)s * kKept + t] - f) <= E;
+            certain = certain && near;
+        }
+        certain = __all_sync(kFullMask, certain);
+    }
+    if (lane == 0) {
+        if (certain) m.status = -1;
+        else atomicAdd(n_open, 1u);
+        open_meta[s] = m;
+    }
+}
+
+__global__ void k_dense_close(const SpecMeta *__restrict__ open_meta, const float *__restrict__ in_s,
+                              const uint64_t *__restrict__ in_k, int32_t nspec, int32_t topn,
+                              const uint32_t *__restrict__ idx_sorted, float *__restrict__ out_s,
+                              uint64_t *__restrict__ out_k, uint32_t *__restrict__ out_pep) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= (int64_t)nspec * topn || open_meta[i / topn].status != 0) return;
+    out_s[i] = in_s[i];
+    out_k[i] = in_k[i];
+    out_pep[i] = in_k[i] != ~0ull ? idx_sorted[in_k[i]] : ~0u;
+}
+
 }  // namespace hfx
 
 using namespace hfx;
@@ -721,5 +822,28 @@ int hfx_dense_score(const uint16_t *lists, uint64_t list_total, const uint32_t *
     if (e != cudaSuccess) return (int)e;
     f<<<sms, kDenseThreads, smem, st>>>(lists, list_total, lstart, total10, list_len, num_pep, tiles, cap_tiles,
                                         (uint32_t)dense_chunks(stride), wb, we, ws.perm, dw, K, stats, err);
+    return (int)cudaGetLastError();
+}
+
+int hfx_dense_prove(const DevDB &db, const SpecMeta *meta, const BatchedWs &ws, const DenseWs &dw, const uint32_t *wb,
+                    const uint32_t *we, const float *rows, int64_t stride, const float *kept_s,
+                    const uint64_t *kept_k, int32_t nspec, int32_t topn, const float *out_s, const uint64_t *out_k,
+                    SpecMeta *open_meta, uint32_t *n_open, cudaStream_t st) {
+    if (topn > 32) return (int)cudaErrorInvalidValue;
+    const cudaError_t e = cudaMemsetAsync(n_open, 0, 4, st);
+    if (e != cudaSuccess) return (int)e;
+    k_dense_ladders<<<dim3((unsigned)dw.cap_blocks, 64), 256, 0, st>>>(db.tc_sorted, db.tn_sorted, dw);
+    k_dense_prove<<<(unsigned)((nspec + 3ll) / 4), 128, 0, st>>>(meta, ws.group_of, ws.groups, dw.blocks, wb, we, rows,
+                                                                 stride, kept_s, kept_k, nspec, topn, out_s, out_k,
+                                                                 open_meta, n_open);
+    return (int)cudaGetLastError();
+}
+
+int hfx_dense_close(const SpecMeta *open_meta, const float *in_s, const uint64_t *in_k, int32_t nspec, int32_t topn,
+                    const uint32_t *idx_sorted, float *out_s, uint64_t *out_k, uint32_t *out_pep, cudaStream_t st) {
+    const int64_t n = (int64_t)nspec * topn;
+    if (n <= 0) return 0;
+    k_dense_close<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(open_meta, in_s, in_k, nspec, topn, idx_sorted, out_s,
+                                                               out_k, out_pep);
     return (int)cudaGetLastError();
 }

@@ -17,6 +17,7 @@ struct DenseBlock {
     int32_t maxlen, charges;
     uint32_t chunk;        // candidates per work item
     uint32_t tile;         // index of its operand tile
+    uint32_t ladder;       // prefixes of its longest candidate (k_dense_ladders)
 };
 
 struct DenseWs {
@@ -57,4 +58,16 @@ int hfx_dense_score(const uint16_t *lists, uint64_t list_total, const uint32_t *
                     const uint16_t *list_len, uint32_t num_pep, const uint8_t *tiles, uint32_t cap_tiles,
                     int64_t stride, int pieces, const uint32_t *wb, const uint32_t *we, int32_t nspec,
                     const hfx::BatchedWs &ws, const hfx::DenseWs &dw, int32_t K, unsigned long long *stats, uint32_t *err,
+                    cudaStream_t st);
+// FP32 searches, after the rescoring: of each spectrum of a dense block, whether
+// its out_s[topn] certainly hold its best candidates (dense.cu).  open_meta: meta
+// with a status other than 0 for every spectrum that needs nothing more;
+// *n_open: how many do.
+int hfx_dense_prove(const hfx::DevDB &db, const hfx::SpecMeta *meta, const hfx::BatchedWs &ws, const hfx::DenseWs &dw,
+                    const uint32_t *wb, const uint32_t *we, const float *rows, int64_t stride, const float *kept_s,
+                    const uint64_t *kept_k, int32_t nspec, int32_t topn, const float *out_s, const uint64_t *out_k,
+                    hfx::SpecMeta *open_meta, uint32_t *n_open, cudaStream_t st);
+// Their results from a plan of the open spectra alone into the search's outputs.
+int hfx_dense_close(const hfx::SpecMeta *open_meta, const float *in_s, const uint64_t *in_k, int32_t nspec,
+                    int32_t topn, const uint32_t *idx_sorted, float *out_s, uint64_t *out_k, uint32_t *out_pep,
                     cudaStream_t st);

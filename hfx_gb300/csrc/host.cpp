@@ -149,6 +149,8 @@ struct hfx_ctx {
     int32_t rows_nspec = 0;
     uint32_t last_items = 0, last_mitems = 0;
     uint32_t last_tiles = 0, cap_tiles = 0, last_ditems = 0, cap_ditems = 0;  // dense blocks: operand tiles, items
+    uint32_t last_open = 0;     // FP32 spectra whose dense results were not certain
+    bool dense_fp32 = true;     // off while a graph is made of a batch that has such spectra
     bool graph_valid = false;
     cudaGraphExec_t graph_exec = nullptr;
     cudaStream_t graph_stream = nullptr;  // captures and replays run here (never the legacy stream)
@@ -639,11 +641,12 @@ int32_t search_batched(hfx_ctx *ctx, const hfx_search_params *p, const Batch &b,
     if (e) return cuda_fail(ctx, e, "alloc");
     // wide windows on the tensor cores: unmodified candidates, lists, up to 32
     // kept, and without a score sink; an FP32 search keeps 32 then and rescores
-    // them, so it has to ask for few enough of them.  A block's pairs are at most
-    // its spectra times their union, so fewer spectra than the rule's share have
-    // no block and need no plan of them (15 us of a one-spectrum search)
+    // them, so it has to ask for few enough of them, and the spectra whose results
+    // are not certain then (hfx_dense_prove) are list-scored below.  A block's pairs
+    // are at most its spectra times their union, so fewer spectra than the rule's
+    // share have no block and need no plan of them (15 us of a one-spectrum search)
     const bool dense_on = lists_only && !long_rows && K <= 32 && p->search_plain != 0 && ns >= kDenseMinPairs &&
-                          (elem_kind != 0 || (p->top_n <= 16 && !ctx->ev_single));
+                          (elem_kind != 0 || (p->top_n <= 16 && !ctx->ev_single && ctx->dense_fp32));
     DenseWs dw{};
     if (dense_on) {
         dw.cap_blocks = dense_blocks(ns);
@@ -937,7 +940,52 @@ int32_t search_batched(hfx_ctx *ctx, const hfx_search_params *p, const Batch &b,
             rc = hfx_ncand(wb, we, meta, ns, plain_on, ncm, out_ncand, ctx->stream);
             if (rc) return cuda_fail(ctx, (cudaError_t)rc, "k_ncand");
         }
-        ctx->stage_end(HFX_STAGE_RESCORE, out_ncand ? 2 : 1, (int64_t)ns * K);
+        int64_t launches = out_ncand ? 2 : 1;
+        if (elem_kind == 0 && dtiles) {
+            SpecMeta *open = ctx->buf<SpecMeta>("d_open", ns, e);
+            if (e) return cuda_fail(ctx, e, "alloc");
+            rc = hfx_dense_prove(db, meta, ws, dw, wb, we, rows, stride, ks, kk, ns, p->top_n, out_s, out_k, open,
+                                 scal + 7, ctx->stream);
+            if (rc) return cuda_fail(ctx, (cudaError_t)rc, "k_dense_prove");
+            launches += 2;
+            if (ctx->gmode >= 1) {
+                // a replay cannot plan them: reported, and the batch searched eagerly
+                rc = hfx_clamp_groups(scal + 7, 0, ctx->d_err.as<uint32_t>(), ctx->stream);
+                if (rc) return cuda_fail(ctx, (cudaError_t)rc, "k_clamp_groups");
+            } else {
+                uint32_t n_open = 0;
+                HFX_CUDA(cudaMemcpyAsync(&n_open, scal + 7, 4, cudaMemcpyDeviceToHost, ctx->stream), "D2H open");
+                HFX_CUDA(cudaStreamSynchronize(ctx->stream), "sync");
+                ctx->last_open = n_open;
+                if (n_open > 0) {
+                    // a plan of these spectra alone over the same lists
+                    rc = hfx_batched_plan(open, ns, wb, we, G, chunk, p->chunk > 0 ? 0 : 1, ws, nullptr, ctx->stream);
+                    if (rc) return cuda_fail(ctx, (cudaError_t)rc, "plan");
+                    uint32_t hs[4];
+                    HFX_CUDA(cudaMemcpyAsync(hs, scal, 16, cudaMemcpyDeviceToHost, ctx->stream), "D2H plan");
+                    HFX_CUDA(cudaStreamSynchronize(ctx->stream), "sync");
+                    K = p->top_n;
+                    tiles = ctx->buf<uint8_t>("tiles", (size_t)hs[1] * stride * G * esz + 64, e);
+                    if (!e) ps = ctx->buf<float>("part_s", (size_t)hs[2] * G * K + 1, e);
+                    if (!e) pk = ctx->buf<uint64_t>("part_k", (size_t)hs[2] * G * K + 1, e);
+                    if (e) return cuda_fail(ctx, e, "alloc parts");
+                    rc = hfx_pack_tiles(src_rows, elem_kind, stride, open, ws, tiles, hs[1], G, ctx->stream);
+                    if (!rc)
+                        rc = hfx_lists_score(lists_out, 0, ctx->d_lstart.as<uint32_t>(), total10_out, llen_out,
+                                             (uint32_t)ctx->num_pep, elem_kind, stride, wb, we, ws, tiles, G, K, 0,
+                                             ps, pk, nullptr, ctx->d_err.as<uint32_t>(), ctx->stream, nullptr,
+                                             nullptr);
+                    if (!rc)
+                        rc = hfx_batched_merge(ps, pk, ws, open, wb, we, ns, G, K, K, ks, kk, nullptr, ctx->stream);
+                    if (!rc)
+                        rc = hfx_dense_close(open, ks, kk, ns, p->top_n, ctx->d_idx.as<uint32_t>(), out_s, out_k,
+                                             out_pep, ctx->stream);
+                    if (rc) return cuda_fail(ctx, (cudaError_t)rc, "open spectra");
+                    launches += (ns <= kSortFew ? 3 : 5) + 4;  // the plan, then these
+                }
+            }
+        }
+        ctx->stage_end(HFX_STAGE_RESCORE, launches, (int64_t)ns * K);
     }
     return HFX_OK;
 }
@@ -1045,11 +1093,19 @@ int32_t search_graph(hfx_ctx *ctx, const hfx_search_params *p, const Batch &b, f
     auto restore = [&](int32_t rc) {
         ctx->gmode = 0;
         ctx->profile = prof;
+        ctx->dense_fp32 = true;
         return rc;
     };
     ctx->gmode = 0;
+    ctx->last_open = 0;
     int32_t rc = search_enqueue(ctx, p, b, out_s, out_k, out_pep, out_ncand);
     if (!rc) rc = search_finish(ctx);
+    if (!rc && ctx->last_open > 0) {
+        // FP32 spectra that need a second plan: a graph of the list scorer alone
+        ctx->dense_fp32 = false;
+        rc = search_enqueue(ctx, p, b, out_s, out_k, out_pep, out_ncand);
+        if (!rc) rc = search_finish(ctx);
+    }
     if (rc) return restore(rc);
     // the group size the eager search used (a requested 16 falls back to 8
     // when more than 32 candidates are kept or the tile does not fit)
