@@ -159,18 +159,24 @@ __device__ __forceinline__ int long_class(uint32_t tc, uint32_t tn, uint32_t nee
 __host__ __device__ constexpr size_t long_bytes(int cls) { return (size_t)long_keys(cls) * 8 + kLongRanges * 4; }
 
 // The bin rint(mz / d), y = RN(1 / d), for the mono or a custom width; from
-// 2^22 on -- beyond every row -- the uncorrected product, which keeps the
+// 2^31 on -- rows are shorter -- the uncorrected product, which keeps the
 // conversion's saturation.
 __device__ __forceinline__ uint32_t bin_long(float mz, float d, float y) {
     const float q = __fmul_rn(mz, y);
-    return __float2uint_rz(q < 4194304.0f ? rintf(quotient(mz, d, y)) : q);
+    return __float2uint_rz(q < 0x1p31f ? rintf(quotient(mz, d, y)) : q);
 }
 
-template <bool FastDiv, int kClass>
+// A key holds the bin, the charge and the level, bin << 4 | (charge - 1) << 2 |
+// level, of rows below 2^28 bins; in longer ones (kWide; a list entry holds 30
+// bits of the bin) it has no charge, and every needed level is sorted by itself.
+constexpr int32_t kNarrowBins = (1 << 28) - 1;
+
+template <bool FastDiv, int kClass, bool kWide>
 __global__ void __launch_bounds__(256) k_gen_lists_long(DevDB db, int32_t nbins, const uint32_t *__restrict__ lstart,
                                                         uint64_t total10, uint32_t *__restrict__ lists,
                                                         uint16_t *__restrict__ list_len, float width, WorkLists wl,
                                                         unsigned long long *__restrict__ stats) {
+    constexpr int kBin = kWide ? 2 : 4;  // the key's bits below the bin
     extern __shared__ __align__(16) uint8_t smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const uint32_t ka = smem_u32(smem) + (uint32_t)warp * (uint32_t)long_bytes(kClass);
@@ -186,19 +192,23 @@ __global__ void __launch_bounds__(256) k_gen_lists_long(DevDB db, int32_t nbins,
     const uint32_t total = wl.count(kClass);
     const uint32_t *work = wl.list(kClass);
     uint32_t my_lists = 0, my_entries = 0, my_res = 0;
-    for (uint32_t t = blockIdx.x * nw + warp; t < total; t += gridDim.x * nw) {
-        const uint32_t p = work[t] & ((1u << kNeedShift) - 1u), need = work[t] >> kNeedShift;
+    constexpr uint32_t kSteps = kWide ? kLevels : 1;  // of a candidate
+    for (uint32_t t = blockIdx.x * nw + warp; t < total * kSteps; t += gridDim.x * nw) {
+        const uint32_t w = work[t / kSteps];
+        const uint32_t p = w & ((1u << kNeedShift) - 1u);
+        const uint32_t need = kWide ? (w >> kNeedShift) & (1u << (t % kSteps)) : w >> kNeedShift;
+        if (kWide && !need) continue;
         const int zmax = 32 - __clz(need);
         const uint32_t tc = db.tc_sorted[p];
         const int len = (int)(db.tn_sorted[p] - tc);
         const float residual = db.r_sorted[p];
         const uint32_t slot = lstart[p];
-        my_res += (uint32_t)len;
+        my_res += kWide && ((w >> kNeedShift) & (need - 1u)) ? 0u : (uint32_t)len;
 #pragma unroll
         for (int i = 0; i < kLongRanges / 128; ++i) sts_u128(cnt + 16u * (uint32_t)(32 * i + lane), make_uint4(0u, 0u, 0u, 0u));
         __syncwarp();
-        // the keys bin << 4 | (charge - 1) << 2 | level (~0: outside the row),
-        // charge by charge, and how many fall into each range
+        // the keys (~0: outside the row), charge by charge, and how many fall
+        // into each range
         float carry = 0.0f;
         for (int k0 = 0; k0 < len; k0 += 32) {
             NoMods mods;
@@ -226,7 +236,8 @@ __global__ void __launch_bounds__(256) k_gen_lists_long(DevDB db, int32_t nbins,
 #pragma unroll
                     for (int j = 0; j < 10; ++j) {
                         const bool in = x[j] < (uint32_t)nbins;
-                        const uint32_t key = x[j] << 4 | (uint32_t)(z - 1) << 2 | (j < 4 ? 1u : (j < 8 ? 2u : 3u));
+                        const uint32_t key = x[j] << kBin | (kWide ? 0u : (uint32_t)(z - 1) << 2) |
+                                             (j < 4 ? 1u : (j < 8 ? 2u : 3u));
                         sts_u32(at + 4u * j, in ? key : ~0u);
                         if (in) red_add(cnt + 4u * (x[j] >> shift), 1u);
                     }
@@ -252,14 +263,14 @@ __global__ void __launch_bounds__(256) k_gen_lists_long(DevDB db, int32_t nbins,
 #pragma unroll 1
         for (int i = lane; i < raw; i += 32) {
             const uint32_t k = lds_u32(ka + 4u * i);
-            if (k != ~0u) sts_u32(kb + 4u * atom_add(cnt + 4u * (k >> (4 + shift)), 1u), k);
+            if (k != ~0u) sts_u32(kb + 4u * atom_add(cnt + 4u * (k >> (kBin + shift)), 1u), k);
         }
         __syncwarp();
         // each key's place within its range
 #pragma unroll 1
         for (int i = lane; i < (int)n; i += 32) {
             const uint32_t k = lds_u32(kb + 4u * i);
-            const uint32_t r = k >> (4 + shift);
+            const uint32_t r = k >> (kBin + shift);
             uint32_t at = r ? lds_u32(cnt + 4u * r - 4u) : 0u;
             const uint32_t end = lds_u32(cnt + 4u * r);
             uint32_t place = at;
@@ -280,15 +291,15 @@ __global__ void __launch_bounds__(256) k_gen_lists_long(DevDB db, int32_t nbins,
             uint32_t best = 0u, bin = ~0u;
             if (i < (int)n) {
                 const uint32_t k = lds_u32(ka + 4u * i);
-                bin = k >> 4;
-                if (i == 0 || (lds_u32(ka + 4u * i - 4u) >> 4) != bin) {
+                bin = k >> kBin;
+                if (i == 0 || (lds_u32(ka + 4u * i - 4u) >> kBin) != bin) {
                     uint32_t o = k;
                     for (int j = i;;) {
-                        const uint32_t c = (o >> 2) & 3u;
+                        const uint32_t c = kWide ? 0u : (o >> 2) & 3u;
                         best = __vmaxu4(best, ((o & 3u) * 0x01010101u) << (8u * c));
                         if (++j >= (int)n) break;
                         o = lds_u32(ka + 4u * j);
-                        if ((o >> 4) != bin) break;
+                        if ((o >> kBin) != bin) break;
                     }
                 }
             }
@@ -879,9 +890,15 @@ int hfx_lists_generate_long(const DevDB &db, const int32_t *cover, int64_t npep1
         f<<<sms * std::max(1, per), nw * 32, smem, st>>>(db, nbins, lstart, total10, lists, list_len, width, wl,
                                                          stats);
     };
-    run(fastdiv ? k_gen_lists_long<true, 1> : k_gen_lists_long<false, 1>, 1, 8);
-    run(fastdiv ? k_gen_lists_long<true, 2> : k_gen_lists_long<false, 2>, 2, 4);
-    run(fastdiv ? k_gen_lists_long<true, 0> : k_gen_lists_long<false, 0>, 0, 2);
+    if (nbins <= kNarrowBins) {
+        run(fastdiv ? k_gen_lists_long<true, 1, false> : k_gen_lists_long<false, 1, false>, 1, 8);
+        run(fastdiv ? k_gen_lists_long<true, 2, false> : k_gen_lists_long<false, 2, false>, 2, 4);
+        run(fastdiv ? k_gen_lists_long<true, 0, false> : k_gen_lists_long<false, 0, false>, 0, 2);
+    } else {
+        run(fastdiv ? k_gen_lists_long<true, 1, true> : k_gen_lists_long<false, 1, true>, 1, 8);
+        run(fastdiv ? k_gen_lists_long<true, 2, true> : k_gen_lists_long<false, 2, true>, 2, 4);
+        run(fastdiv ? k_gen_lists_long<true, 0, true> : k_gen_lists_long<false, 0, true>, 0, 2);
+    }
     return (int)cudaGetLastError();
 }
 
