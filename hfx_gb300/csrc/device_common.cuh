@@ -684,12 +684,20 @@ struct WarpTopK {
     }
 };
 
+// `better` as a strict order of all scores, NaN first: both lanes of an exchange
+// have to agree which entry is whose, or one of the two is lost.
+__device__ __forceinline__ bool before(float sa, uint64_t ka, float sb, uint64_t kb) {
+    if (sa > sb || sa < sb) return sa > sb;
+    const bool na = sa != sa, nb = sb != sb;
+    return na != nb ? na : ka < kb;
+}
+
 // Compare-exchange with lane ^ d, the better entry to the lower lane.
 __device__ __forceinline__ void better_first(float &s, uint64_t &k, int d) {
     const float os = __shfl_xor_sync(kFullMask, s, d);
     const uint64_t ok = __shfl_xor_sync(kFullMask, k, d);
     const bool lower = ((threadIdx.x & 31) & d) == 0;
-    if (better(os, ok, s, k) == lower) {
+    if (before(os, ok, s, k) == lower) {
         s = os;
         k = ok;
     }
@@ -711,7 +719,7 @@ struct WarpList32 {
         const int lane = threadIdx.x & 31;
         const float rs = __shfl_sync(kFullMask, os, 31 - lane);
         const uint64_t rk = __shfl_sync(kFullMask, ok, 31 - lane);
-        if (better(rs, rk, s, k)) {
+        if (before(rs, rk, s, k)) {
             s = rs;
             k = rk;
         }
@@ -746,15 +754,15 @@ struct WarpList64 {
         const int i1 = 63 - lane, i0 = 31 - lane;
         const float a = i1 < n ? ps[i1] : -INFINITY, b = i0 < n ? ps[i0] : -INFINITY;
         const uint64_t ka = i1 < n ? pk[i1] : ~0ull, kb = i0 < n ? pk[i0] : ~0ull;
-        if (better(a, ka, s0, k0)) {
+        if (before(a, ka, s0, k0)) {
             s0 = a;
             k0 = ka;
         }
-        if (better(b, kb, s1, k1)) {
+        if (before(b, kb, s1, k1)) {
             s1 = b;
             k1 = kb;
         }
-        if (better(s1, k1, s0, k0)) {
+        if (before(s1, k1, s0, k0)) {
             const float ts = s0;
             const uint64_t tk = k0;
             s0 = s1;

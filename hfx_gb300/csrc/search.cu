@@ -115,7 +115,9 @@ __global__ void __launch_bounds__(256) k_score_spectra(DevDB db, const float *__
     }
 }
 
-// Merge per-spectrum partial lists into the final top-N, a block each.
+// Merge per-spectrum partial lists into the final top-N, a block each.  Lists that
+// hold a NaN (of an infinite intensity's bin) have no order to merge by: their
+// entries are inserted one by one.
 constexpr int kPartWarps = 4;
 __global__ void __launch_bounds__(32 * kPartWarps) k_merge_parts(const float *__restrict__ part_s, const uint64_t *__restrict__ part_k,
                               const int64_t *__restrict__ part_off, int32_t nspec, int32_t K, int32_t topn,
@@ -127,12 +129,24 @@ __global__ void __launch_bounds__(32 * kPartWarps) k_merge_parts(const float *__
     __shared__ uint64_t sm_k[kPartWarps][32];
     WarpList32 tk;
     tk.init();
-    for (int64_t b = part_off[s] + warp; b < part_off[s + 1]; b += kPartWarps)
-        tk.merge_list(part_s + b * K, part_k + b * K, K);
+    bool nan = false;
+    for (int64_t b = part_off[s] + warp; b < part_off[s + 1]; b += kPartWarps) {
+        const float ps = lane < K ? part_s[b * K + lane] : -INFINITY;
+        nan |= ps != ps;
+        tk.merge(ps, lane < K ? part_k[b * K + lane] : ~0ull);
+    }
     if (warp > 0) tk.store(sm_s[warp], sm_k[warp], 32);
-    __syncthreads();
+    nan = __syncthreads_or(nan);
     if (warp > 0) return;
-    for (int w = 1; w < kPartWarps; ++w) tk.merge_list(sm_s[w], sm_k[w], 32);
+    for (int w = 1; w < kPartWarps && !nan; ++w) tk.merge_list(sm_s[w], sm_k[w], 32);
+    if (nan) {
+        WarpTopK one;
+        one.init();
+        for (int64_t j = part_off[s] * K; j < part_off[s + 1] * K; ++j)
+            if (part_k[j] != ~0ull) one.insert(part_s[j], part_k[j], topn);
+        tk.s = one.s;
+        tk.k = one.k;
+    }
     if (lane < topn) {
         out_s[(size_t)s * topn + lane] = tk.s;
         out_k[(size_t)s * topn + lane] = tk.k;
