@@ -81,14 +81,17 @@ __host__ __device__ __forceinline__ uint32_t swizzled(uint32_t r, uint32_t k) {
 // and open windows have 36 to 115 (kDenseMinPairs).
 constexpr uint32_t kDenseMinWidth = 4096;
 
-// One warp per block.  Classes as in k_groups.
 __global__ void k_dense_clear(DenseWs dw, int32_t nspec) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < 32ll * nspec) dw.best[i] = 0ull;
-    if (i < nspec) dw.thr[i] = dw.lock[i] = 0u;
+    if (i < nspec) {
+        dw.thr[i] = 0u;
+        dw.lock[i] = i == 0 && (*dw.hold & 0xFFu) ? 2u : 0u;
+    }
     if (i == 0) *dw.n_tiles = *dw.counter = dw.item_off[dw.cap_blocks] = 0u;
 }
 
+// One warp per block.  Classes as in k_groups.
 __global__ void k_dense_plan(const SpecMeta *__restrict__ meta, const uint32_t *__restrict__ wb,
                              const uint32_t *__restrict__ we, int32_t G, const uint32_t *__restrict__ bucket_end,
                              int32_t nclass, int32_t nbucket, const int32_t *__restrict__ perm,
@@ -280,6 +283,7 @@ struct DenseBars {
     uint64_t piece_full[kPieceStages], piece_empty[kPieceStages];  // the spectra's pieces
     uint64_t rows_full[2], rows_empty[2];                          // the candidates' weights
     uint64_t acc_full, acc_empty;                                  // the accumulators
+    uint64_t drain;                                                // MMAs in flight when a wait gave up
 };
 
 constexpr uint32_t kDenseWaitLimit = 1u << 21;
@@ -292,6 +296,21 @@ __device__ __forceinline__ bool dense_wait(uint64_t *bar, uint32_t phase, volati
     }
     *give_up = 1u;
     atomicOr(err, kErrTimeout);
+    return false;
+}
+// The same for a whole warp: every lane polls, and so sees what the phase
+// publishes, and all lanes go on or all give up -- the warp-wide steps that
+// follow need every lane.
+__device__ __forceinline__ bool dense_wait_warp(uint64_t *bar, uint32_t phase, volatile uint32_t *give_up,
+                                                uint32_t *err) {
+    for (uint32_t i = 0; i < kDenseWaitLimit; ++i) {
+        if (__all_sync(kFullMask, mbar_wait(bar, phase, 1u))) return true;
+        if ((i & 63u) == 63u && __any_sync(kFullMask, *give_up != 0u)) return false;
+    }
+    if ((threadIdx.x & 31) == 0) {
+        *give_up = 1u;
+        atomicOr(err, kErrTimeout);
+    }
     return false;
 }
 __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
@@ -329,6 +348,7 @@ k_dense_score(const uint16_t *__restrict__ lists, uint64_t list_total, const uin
         }
         mbar_init(&bar.acc_full, 1);
         mbar_init(&bar.acc_empty, 4);
+        mbar_init(&bar.drain, 1);
         s_give_up = 0u;
     }
     if (warp == kSpreadWarps + 4) {  // the MMA warp owns the tensor memory
@@ -382,7 +402,11 @@ k_dense_score(const uint16_t *__restrict__ lists, uint64_t list_total, const uin
             }
         uint32_t got = 0u;
         if (lane == 0)
-            for (uint32_t i = 0; i < kLockLimit && !got; ++i) got = atomicCAS(dw.lock + sj, 0u, 1u) == 0u;
+            for (uint32_t i = 0; i < kLockLimit && !got; ++i) {
+                got = atomicCAS(dw.lock + sj, 0u, 1u) == 0u;
+                // the search has failed already: the other locks need not run out too
+                if ((i & 255u) == 255u && (*(volatile uint32_t *)err & kErrTimeout)) break;
+            }
         got = __shfl_sync(kFullMask, got, 0);
         if (!got) {
             if (lane == 0) atomicOr(err, kErrTimeout);
@@ -466,7 +490,7 @@ k_dense_score(const uint16_t *__restrict__ lists, uint64_t list_total, const uin
                 for (int i = 0; i < kWindow; ++i) v[i] = load8(8u * i);
                 for (uint32_t c = 0; c < chunks; ++c, ++n_chunk) {
                     const uint32_t buf = n_chunk & 1u;
-                    if (!dense_wait(&bar.rows_empty[buf], ((n_chunk >> 1) & 1u) ^ 1u, &s_give_up, err)) goto done;
+                    if (!dense_wait_warp(&bar.rows_empty[buf], ((n_chunk >> 1) & 1u) ^ 1u, &s_give_up, err)) goto done;
                     const uint32_t row = row0 + buf * kDenseChunkBytes;
 #pragma unroll
                     for (uint32_t j = 0; j < 8; ++j) sts_u128(row + ((j ^ sw) << 4), make_uint4(0u, 0u, 0u, 0u));
@@ -533,7 +557,7 @@ k_dense_score(const uint16_t *__restrict__ lists, uint64_t list_total, const uin
             }
             for (uint32_t pass = 0; pass < passes; ++pass, ++n_pass) {
                 if (s >= 0) thr = fmaxf(thr, score_of(__ldcg(dw.thr + s)));
-                if (!dense_wait(&bar.acc_full, n_pass & 1u, &s_give_up, err)) goto done;
+                if (!dense_wait_warp(&bar.acc_full, n_pass & 1u, &s_give_up, err)) goto done;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t pb = p0 + pass * kDenseRows;
                 const uint32_t pe = min(p1, pb + kDenseRows);
@@ -659,9 +683,8 @@ k_dense_score(const uint16_t *__restrict__ lists, uint64_t list_total, const uin
             for (uint32_t i = n_piece > kPieceStages ? n_piece - kPieceStages : 0u; i < n_piece; ++i)
                 mbar_wait(&bar.piece_full[i % kPieceStages], (i / kPieceStages) & 1u, kDenseWaitLimit);
         if (warp == kSpreadWarps + 4 && lane == 0) {
-            mbar_init(&bar.acc_full, 1);
-            mma_commit(smem_u32(&bar.acc_full));
-            mbar_wait(&bar.acc_full, 0u, kDenseWaitLimit);
+            mma_commit(smem_u32(&bar.drain));
+            mbar_wait(&bar.drain, 0u, kDenseWaitLimit);
         }
         __syncwarp();
     }

@@ -660,6 +660,7 @@ int32_t search_batched(hfx_ctx *ctx, const hfx_search_params *p, const Batch &b,
         dw.n_tiles = scal + 4;
         dw.total_items = scal + 5;
         dw.counter = scal + 6;
+        dw.hold = ctx->d_err.as<uint32_t>() + 1;
     }
     ws.n_sorted = scal;
     ws.ngroups = scal + 1;
@@ -993,7 +994,9 @@ int32_t search_batched(hfx_ctx *ctx, const hfx_search_params *p, const Batch &b,
 // Failure-detection test: HFX_TEST_HOLD_LOCK=1 makes every scorer CTA start
 // with member 0's admission lock held by nobody, so each merge into it gives
 // up after its bounded number of attempts (2^20), the CTA records a timeout
-// in the error word and goes on, and the search returns HFX_ERR_TIMEOUT.
+// in the error word and goes on, and the search returns HFX_ERR_TIMEOUT.  The
+// tensor-core blocks start with the first spectrum's list locked, and the waits
+// of a CTA that hangs on it run out as well.
 // Read at each search (eager searches; a captured graph keeps the value of
 // its capture).  Off (0) by default.
 int test_lock_attempts() {
