@@ -63,6 +63,7 @@ bool cleaves_after(int rule, uint8_t c) {  // Config.hs:415-431
 struct DBuf {
     void *p = nullptr;
     size_t n = 0;
+    bool in_graph = false;  // the captured graph holds its address
     cudaError_t ensure(size_t bytes) {
         if (bytes <= n) return cudaSuccess;
         if (p) cudaFree(p);
@@ -161,6 +162,7 @@ struct hfx_ctx {
         graph_exec = nullptr;
         graph_valid = false;
         graph_key.clear();
+        for (auto &kv : ws) kv.second.in_graph = false;
     }
 
     // HFX_DEBUG_SYNC=1: synchronize after every stage and remember the first
@@ -220,6 +222,7 @@ struct hfx_ctx {
     void drop(const char *name) {
         auto it = ws.find(name);
         if (it == ws.end()) return;
+        if (it->second.in_graph) graph_reset();
         it->second.release();
         ws.erase(it);
     }
@@ -230,6 +233,10 @@ struct hfx_ctx {
             e = cudaErrorMemoryAllocation;
             return nullptr;
         }
+        // a graph's kernels keep the addresses of its capture: one whose
+        // workspace moves is not replayed again
+        if (gmode == 2) b.in_graph = true;
+        else if (want > b.n && b.in_graph) graph_reset();
         e = b.ensure(want);
         return b.as<T>();
     }
