@@ -152,12 +152,10 @@ __global__ void __launch_bounds__(kSortFew) k_sort_few(const SpecMeta *__restric
 }
 
 // With few_groups (no work-item size asked for) a group's window is cut so
-// that about this many items come of all groups together, four per resident
+// that about kFewItems items come of all groups together, four per resident
 // CTA of the list scorer: one spectrum's 3,400 candidates in one item kept one
 // SM busy for 0.22 ms.  Groups of narrow and of wide windows count apart; from
 // about 1,200 groups (76 of open windows) on the rule changes nothing.
-constexpr uint32_t kFewItems = 1216;
-
 // One thread per group: members, union window, chunk count.
 // bucket_end[b] = end of bucket b's spectra in sorted order (the scanned
 // counters, which the scatter has moved from the starts to the ends).

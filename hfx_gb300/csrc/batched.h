@@ -28,6 +28,9 @@ struct BatchedWs {
 
 constexpr int kBucketCount = 12 * 8192;
 constexpr int kSortFew = 1024;      // spectra that one block sorts without the buckets
+// Work items that the planning cuts few groups' windows into, of narrow and of
+// wide windows each (k_groups).
+constexpr uint32_t kFewItems = 1216;
 struct DenseWs;
 }  // namespace hfx
 

@@ -1097,7 +1097,11 @@ int32_t search_graph(hfx_ctx *ctx, const hfx_search_params *p, const Batch &b, f
         const int32_t rc = search_finish(ctx, &herr);
         if (!(herr & (kErrBounds | kErrTooLong))) return rc;
     }
-    ctx->graph_reset();  // no graph yet, another shape, or the batch outgrew the capture
+    // no graph yet, another shape, or the batch outgrew the capture: the new one
+    // then has room for both, or batches that need more of one kind of work and
+    // less of another would be planned again in turn
+    const bool outgrown = ctx->graph_valid && key == ctx->graph_key;
+    ctx->graph_reset();
     const bool prof = ctx->profile;
     ctx->profile = false;
     auto restore = [&](int32_t rc) {
@@ -1122,9 +1126,19 @@ int32_t search_graph(hfx_ctx *ctx, const hfx_search_params *p, const Batch &b, f
     const int32_t G = ctx->last_G > 0 ? ctx->last_G : (p->precision == 0 ? 4 : 8);
     ctx->cap_stride = ctx->last_stride;
     ctx->cap_groups = (uint32_t)((b.nspec + G - 1) / G + 24);  // <= one partial group per class
-    ctx->cap_items = ctx->last_items + ctx->last_items / 4 + 64;
-    ctx->cap_tiles = ctx->last_tiles ? ctx->last_tiles + ctx->last_tiles / 4 + 2 : 0;
-    ctx->cap_ditems = ctx->last_ditems ? ctx->last_ditems + ctx->last_ditems / 4 + 64 : 0;
+    // few groups have more items the wider their windows are, up to kFewItems of
+    // each kind beyond what the work-item size alone gives
+    uint32_t items = ctx->last_items + ctx->last_items / 4 + 64 + (p->chunk > 0 ? 0u : 2u * kFewItems);
+    uint32_t tiles = ctx->last_tiles ? ctx->last_tiles + ctx->last_tiles / 4 + 2 : 0;
+    uint32_t ditems = ctx->last_ditems ? ctx->last_ditems + ctx->last_ditems / 4 + 64 : 0;
+    if (outgrown) {
+        items = std::max(items, ctx->cap_items);
+        tiles = std::max(tiles, ctx->cap_tiles);
+        ditems = std::max(ditems, ctx->cap_ditems);
+    }
+    ctx->cap_items = items;
+    ctx->cap_tiles = tiles;
+    ctx->cap_ditems = ditems;
     ctx->cap_mitems = ctx->last_mitems + ctx->last_mitems / 4 + 64;
     ctx->cap_iso = ctx->last_iso + ctx->last_iso / 4 + 64;
     ctx->cap_iso_entries = ctx->last_iso_entries + ctx->last_iso_entries / 4 + 4096;
