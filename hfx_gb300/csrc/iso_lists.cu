@@ -638,7 +638,9 @@ int hfx_iso_generate(const DevDB &db, const DevMods &m, const int32_t *cover, in
         db, m, total_p, cap_iso, iso_key, pos_words, iso_pos, wl, iso_len, err);
     auto run = [&](auto f, int cls) {
         const size_t smem = (size_t)(256 / class_lanes(cls)) * rank_bytes(nbins, cls);
-        cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        // (the longest rows': see hfx_lists_generate)
+        cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)((256 / class_lanes(cls)) * rank_bytes(kMaxWords * 32, cls)));
         int per = 0;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, f, 256, smem);
         f<<<sms * std::max(1, cls ? per : std::min(per, 2)), 256, smem, st>>>(

@@ -747,7 +747,9 @@ int hfx_lists_generate(const DevDB &db, const int32_t *cover, int64_t npep1, int
     k_list_work<false><<<(db.num_pep + 255) / 256, 256, 0, st>>>(db, cover, npep1, list_len, wl, nullptr);
     auto run = [&](auto f, int cls) {
         const size_t smem = (size_t)(256 / class_lanes(cls)) * rank_bytes(nbins, cls);
-        cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        // the limit is the function's, common to all contexts and threads: that of the longest rows
+        cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)((256 / class_lanes(cls)) * rank_bytes(kMaxWords * 32, cls)));
         int per = 0;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, f, 256, smem);
         f<<<sms * std::max(1, cls ? per : std::min(per, 2)), 256, smem, st>>>(db, nbins, lstart, total10, lists,

@@ -241,7 +241,10 @@ int hfx_launch_score_spectra(const DevDB &db, const float *rows, int64_t stride,
     if (nblocks <= 0) return 0;
     const size_t smem = score_smem_bytes((int32_t)stride, words, nw, K);
     auto f = fastdiv ? k_score_spectra<true> : k_score_spectra<false>;
-    cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // the limit is the function's, common to all contexts and threads: that of the longest rows
+    const cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)score_smem_bytes(kMaxWords * 32, kMaxWords, nw, kMaxTopK));
+    if (e != cudaSuccess) return (int)e;
     f<<<(unsigned)nblocks, nw * 32, smem, st>>>(db, rows, stride, meta, wb, we, part_off, nspec, K, part_s, part_k);
     return (int)cudaGetLastError();
 }
