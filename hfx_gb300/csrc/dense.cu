@@ -85,7 +85,7 @@ __global__ void k_dense_clear(DenseWs dw, int32_t nspec) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < 32ll * nspec) dw.best[i] = 0ull;
     if (i < nspec) {
-        dw.thr[i] = 0u;
+        dw.kth[i] = 0ull;
         dw.lock[i] = i == 0 && (*dw.hold & 0xFFu) ? 2u : 0u;
     }
     if (i == 0) *dw.n_tiles = *dw.counter = dw.item_off[dw.cap_blocks] = 0u;
@@ -380,12 +380,20 @@ k_dense_score(const uint16_t *__restrict__ lists, uint64_t list_total, const uin
     // counts give the buffer and the barrier phase
     uint32_t n_chunk = 0, n_piece = 0, n_pass = 0;
     unsigned long long my_rows = 0, my_entries = 0, my_pairs = 0;
-    // epilogue warps: the item's spectrum of this lane, its window, its
-    // threshold and its queue
+    // epilogue warps: the item's spectrum of this lane, its window, the key that
+    // a candidate has to exceed (its list's K-th) and its queue.  Spectra of a few
+    // peaks have thousands of candidates tied with the K-th: those behind it are
+    // not looked at (cut), or the merging of them would take ten times the rest
     const uint32_t m = threadIdx.x & (kDenseSpectra - 1u);
     int32_t s = -1;
     uint32_t a = 0, e = 0, qn = 0;
-    float thr = INFINITY;
+    unsigned long long floor_key = ~0ull;
+    // the least score that is kept at positions from p on
+    auto cut_from = [&](uint32_t p) {
+        const uint32_t order = (uint32_t)(floor_key >> 32);
+        if (order == ~0u) return INFINITY;
+        return score_of(order + (order != 0u && (uint32_t)~(uint32_t)floor_key < p ? 1u : 0u));
+    };
     // Merges lane j's queue into its spectrum's list (warp-wide).
     auto merge = [&](int j) {
         const int cnt = (int)__shfl_sync(kFullMask, qn, j);
@@ -423,14 +431,14 @@ k_dense_score(const uint16_t *__restrict__ lists, uint64_t list_total, const uin
             l = (lane & o) == 0 ? max(l, y) : min(l, y);
         }
         __stcg(list + lane, l);
-        const uint32_t kth = (uint32_t)(__shfl_sync(kFullMask, l, K - 1) >> 32);
-        if (lane == 0) __stcg(dw.thr + sj, kth);
+        const unsigned long long kth = __shfl_sync(kFullMask, l, K - 1);
+        if (lane == 0) __stcg(dw.kth + sj, kth);
         __threadfence();
         __syncwarp();
         if (lane == 0) atomicExch(dw.lock + sj, 0u);
         if (lane == j) {
             qn = 0;
-            thr = fmaxf(thr, score_of(kth));
+            floor_key = max(floor_key, kth);
         }
         __syncwarp();
     };
@@ -545,18 +553,18 @@ k_dense_score(const uint16_t *__restrict__ lists, uint64_t list_total, const uin
         } else if (warp < kSpreadWarps + 4) {
             // ---- accumulators -> the best K: lane = spectrum ----
             // Full queues are merged into the spectrum's list in global memory
-            // (sorted, under a lock), whose K-th score is the threshold of
-            // every CTA.  (A list per item started anew every 8,192 candidates:
+            // (sorted, under a lock), whose K-th is the threshold of every
+            // CTA.  (A list per item started anew every 8,192 candidates:
             // 100,000 cycles of merging a pass.)
             {
                 s = m < d.count ? perm[d.pos0 + m] : -1;
                 a = s >= 0 ? wb[s] : 0u;
                 e = s >= 0 ? we[s] : 0u;
-                thr = s >= 0 ? -INFINITY : INFINITY;
+                floor_key = s >= 0 ? 0ull : ~0ull;
                 qn = 0;
             }
             for (uint32_t pass = 0; pass < passes; ++pass, ++n_pass) {
-                if (s >= 0) thr = fmaxf(thr, score_of(__ldcg(dw.thr + s)));
+                if (s >= 0) floor_key = max(floor_key, __ldcg(dw.kth + s));
                 if (!dense_wait_warp(&bar.acc_full, n_pass & 1u, &s_give_up, err)) goto done;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t pb = p0 + pass * kDenseRows;
@@ -566,7 +574,7 @@ k_dense_score(const uint16_t *__restrict__ lists, uint64_t list_total, const uin
                 const uint32_t acc = tmem + ((m >> 5) << 21);
                 // no threshold yet: the largest of nine cuts between the lowest
                 // and the highest score that at least K of this pass reach
-                const bool fresh = s >= 0 && thr == -INFINITY && c1 >= c0 + (uint32_t)K;
+                const bool fresh = floor_key == 0ull && c1 >= c0 + (uint32_t)K;
                 if (__any_sync(kFullMask, fresh)) {
                     float low = INFINITY, high = -INFINITY;
                     float v[32];
@@ -593,7 +601,7 @@ k_dense_score(const uint16_t *__restrict__ lists, uint64_t list_total, const uin
                         if (n >= (uint32_t)K) low = cut;
                         else high = cut;
                     }
-                    if (fresh) thr = low;
+                    if (fresh) floor_key = (unsigned long long)score_order(low) << 32;
                 }
 #pragma unroll 1
                 for (uint32_t j0 = 0; j0 < kDenseRows; j0 += 32) {
@@ -604,17 +612,18 @@ k_dense_score(const uint16_t *__restrict__ lists, uint64_t list_total, const uin
                     for (int j = 1; j < 30; j += 2) top = max_nan(top, v[j], v[j + 1]);
                     // this spectrum's columns of these 32
                     const uint32_t from = c0 > j0 ? min(c0 - j0, 32u) : 0u, to = c1 > j0 ? min(c1 - j0, 32u) : 0u;
-                    if (!__any_sync(kFullMask, to > from && !(top < thr))) continue;
+                    const float cut = cut_from(pb + j0);
+                    if (!__any_sync(kFullMask, to > from && !(top < cut))) continue;
                     uint32_t hit = 0;
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) hit |= v[j] < thr ? 0u : 1u << j;
+                    for (int j = 0; j < 32; ++j) hit |= v[j] < cut ? 0u : 1u << j;
                     hit &= to > from ? (0xFFFFFFFFu >> (32u - (to - from))) << from : 0u;
                     // the columns some lane keeps, one at a time (read again: a
                     // register is not indexed by a column)
                     for (uint32_t any = __reduce_or_sync(kFullMask, hit); any; any &= any - 1u) {
                         const uint32_t j = (uint32_t)__ffs(any) - 1u;
-                        const float x = tmem_load1(acc + j0 + j);
-                        if ((hit >> j) & 1u) q[m * kDenseQueue + qn++] = packed(x, pb + j0 + j);
+                        const unsigned long long x = packed(tmem_load1(acc + j0 + j), pb + j0 + j);
+                        if (((hit >> j) & 1u) && x > floor_key) q[m * kDenseQueue + qn++] = x;
                         uint32_t full = __ballot_sync(kFullMask, qn == (uint32_t)kDenseQueue);
                         __syncwarp();
                         while (full) {

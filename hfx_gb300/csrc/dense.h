@@ -30,7 +30,7 @@ struct DenseWs {
     unsigned long long *best;  // [nspec][32] each spectrum's best candidates so far, descending: score order << 32 | ~position
     unsigned long long *left;  // [items][128][kDenseQueue] candidates an item did not merge into it (0: none)
     uint32_t *lock;        // [nspec] of that list
-    uint32_t *thr;         // [nspec] its K-th score (ordered bits, 0 = none yet)
+    unsigned long long *kth;  // [nspec] its K-th entry (0: none yet)
     const uint32_t *hold;  // failure test: not 0: the first spectrum's lock starts held by nobody
     int32_t cap_blocks;
 };

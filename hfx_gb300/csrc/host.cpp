@@ -660,7 +660,7 @@ int32_t search_batched(hfx_ctx *ctx, const hfx_search_params *p, const Batch &b,
         dw.blocks = ctx->buf<DenseBlock>("d_blocks", dw.cap_blocks, e);
         dw.item_off = e ? nullptr : ctx->buf<uint32_t>("d_itemoff", (size_t)dw.cap_blocks + 1, e);
         dw.tile_block = e ? nullptr : ctx->buf<uint32_t>("d_tileblock", dw.cap_blocks, e);
-        dw.thr = e ? nullptr : ctx->buf<uint32_t>("d_thr", ns, e);
+        dw.kth = e ? nullptr : ctx->buf<unsigned long long>("d_kth", ns, e);
         dw.lock = e ? nullptr : ctx->buf<uint32_t>("d_lock", ns, e);
         dw.best = e ? nullptr : ctx->buf<unsigned long long>("d_best", 32ull * ns, e);
         if (e) return cuda_fail(ctx, e, "alloc");
