@@ -218,6 +218,27 @@ struct hfx_ctx {
         for (const auto &kv : ws) t += kv.second.n;
         return t;
     }
+    // A search that finds no room is done once more in the least room: without
+    // what helps speed alone -- tensor-core tiles and queues, the smaller items and
+    // groups of the planning, the isoforms' lists of work -- and with no workspace
+    // that an earlier search left larger.
+    bool lean = false;
+    void drop_search_workspaces() {
+        if (stream) cudaStreamSynchronize(stream);
+        if (graph_stream) cudaStreamSynchronize(graph_stream);
+        graph_reset();
+        for (auto it = ws.begin(); it != ws.end();) {
+            // (the inputs and outputs of hfx_search_host stay)
+            if (it->first.compare(0, 3, "in_") == 0 || it->first.compare(0, 4, "out_") == 0) {
+                ++it;
+                continue;
+            }
+            it->second.release();
+            it = ws.erase(it);
+        }
+        rows_nspec = 0;
+        cudaGetLastError();  // a failed allocation's
+    }
     // Frees a workspace (one-time scratch such as the digest's).
     void drop(const char *name) {
         auto it = ws.find(name);
@@ -571,16 +592,26 @@ int32_t search_isoform_lists(hfx_ctx *ctx, const hfx_search_params *p, const Spe
     uint16_t *lists = e ? nullptr : ctx->buf<uint16_t>("i_lists", cap_entries + 64, e);
     const int32_t pos_words = (int32_t)((ctx->max_ladder + 31) / 32 + 1);
     uint32_t *pos = e ? nullptr : ctx->buf<uint32_t>("i_pos", (cap_iso + 1) * (size_t)pos_words, e);
-    uint32_t *work = e ? nullptr : ctx->buf<uint32_t>("i_work", hfx_lists_work_words(cap_iso), e);
+    // the lists of work: where there is little room, in the place of the isoforms'
+    // list sizes, which nothing reads after the expansion, some records at a time
+    uint64_t work_cap = ctx->lean ? std::min(cap_iso, hfx_lists_work_cap(2 * (uint64_t)n)) : 0;
+    uint32_t *work = reinterpret_cast<uint32_t *>(units);
+    if (work_cap == 0) {
+        work_cap = cap_iso;
+        work = e ? nullptr : ctx->buf<uint32_t>("i_work", hfx_lists_work_words(work_cap), e);
+    }
     if (e) return cuda_fail(ctx, e, "alloc isoform lists");
     rc = hfx_iso_expand(db, dm, cover, ctx->d_lstart.as<uint32_t>(), count, incl, units, iunits, (uint32_t)cap_iso,
                         cap_entries, key, off, ctx->d_err.as<uint32_t>(), ctx->stream);
     if (!rc)
         rc = hfx_iso_generate(db, dm, cover, (int32_t)std::min<int64_t>(stride, kMaxWords * 32),
                               ctx->d_lstart.as<uint32_t>(), incl + n, (uint32_t)cap_iso, key, off, lists, cap_entries,
-                              len, pos_words, pos, work, p->fastdiv, stats, ctx->d_err.as<uint32_t>(), ctx->stream);
+                              len, pos_words, pos, work, work_cap, p->fastdiv, stats, ctx->d_err.as<uint32_t>(),
+                              ctx->stream);
     if (rc) return cuda_fail(ctx, (cudaError_t)rc, "isoform lists");
-    ctx->stage_end(HFX_STAGE_MOD_LISTS, 19, (int64_t)cap_iso);  // windows, planning, 14 isoform-list kernels
+    // windows, planning, 9 isoform-list kernels and 5 for each run of records
+    ctx->stage_end(HFX_STAGE_MOD_LISTS, 14 + 5 * (int64_t)((cap_iso + work_cap - 1) / std::max<uint64_t>(work_cap, 1)),
+                   (int64_t)cap_iso);
     ctx->stage_begin(HFX_STAGE_MODS);
     rc = hfx_iso_score(lists, cap_entries, ctx->d_lstart.as<uint32_t>(), key, off, len, count, incl,
                        (uint32_t)ctx->num_pep, (uint32_t)cap_iso, elem_kind, tiles, stride, mb, me, ctx->num_mod, ws,
@@ -606,11 +637,12 @@ int32_t search_batched(hfx_ctx *ctx, const hfx_search_params *p, const Batch &b,
     // 8 on average with 2,000 spectra): two of the smaller tiles fit an SM, and
     // the scorer took 14.0 against 22 ms (FP32, 1,000 spectra: 2.6 against 3.5)
     const bool iso = p->batch_mode == 1 && p->search_mods != 0 && ctx->num_mod > 0;
-    int32_t G = p->group_size > 0 ? p->group_size : (elem_kind == 0 ? 4 : 8) / (iso ? 2 : 1);
+    int32_t G = p->group_size > 0 ? p->group_size : (elem_kind == 0 ? 4 : 8) / (iso && !ctx->lean ? 2 : 1);
     // no member that the batch does not have (one spectrum of open windows: 1.01 ->
     // 0.94 ms; BF16 isoforms are slower so, 1.74 -> 1.86 ms)
     while (p->group_size <= 0 && !iso && G > 1 && G / 2 >= ns) G /= 2;
     const int32_t chunk = p->chunk > 0 ? p->chunk : 4096;
+    const int few_groups = p->chunk > 0 || ctx->lean ? 0 : 1;
     if (G != 1 && G != 2 && G != 4 && G != 8 && G != 16)
         return fail(ctx, HFX_ERR_ARG, "group_size must be 1, 2, 4, 8 or 16");
     // rows longer than the shared-memory bit planes: 32-bit sorted lists,
@@ -653,7 +685,7 @@ int32_t search_batched(hfx_ctx *ctx, const hfx_search_params *p, const Batch &b,
     // are at most its spectra times their union, so fewer spectra than the rule's
     // share have no block and need no plan of them (15 us of a one-spectrum search)
     const bool dense_on = lists_only && !long_rows && K <= 32 && p->search_plain != 0 && ns >= kDenseMinPairs &&
-                          (elem_kind != 0 || (p->top_n <= 16 && !ctx->ev_single && ctx->dense_fp32));
+                          !ctx->lean && (elem_kind != 0 || (p->top_n <= 16 && !ctx->ev_single && ctx->dense_fp32));
     DenseWs dw{};
     if (dense_on) {
         dw.cap_blocks = dense_blocks(ns);
@@ -686,8 +718,7 @@ int32_t search_batched(hfx_ctx *ctx, const hfx_search_params *p, const Batch &b,
     ctx->stage_begin(HFX_STAGE_WINDOWS);
     int rc = hfx_launch_windows(ctx->d_r.as<float>(), (uint32_t)ctx->num_pep, meta, ns, wb, we, ctx->stream);
     if (rc) return cuda_fail(ctx, (cudaError_t)rc, "k_windows");
-    rc = hfx_batched_plan(meta, ns, wb, we, G, chunk, p->chunk > 0 ? 0 : 1, ws, dense_on ? &dw : nullptr,
-                          ctx->stream);
+    rc = hfx_batched_plan(meta, ns, wb, we, G, chunk, few_groups, ws, dense_on ? &dw : nullptr, ctx->stream);
     if (rc) return cuda_fail(ctx, (cudaError_t)rc, "plan");
     // k_windows + the planning kernels
     ctx->stage_end(HFX_STAGE_WINDOWS, (dense_on ? 8 : 6) - (ns <= kSortFew ? 2 : 0), ns);
@@ -766,8 +797,6 @@ int32_t search_batched(hfx_ctx *ctx, const hfx_search_params *p, const Batch &b,
     } else {
         // lists: one ion list per needed (peptide, charge level), then scoring
         const int64_t npep1 = (int64_t)ctx->num_pep + 1;
-        int32_t *diff = ctx->buf<int32_t>("l_diff", (size_t)kLevels * npep1, e);
-        if (e) return cuda_fail(ctx, e, "alloc");
         int32_t *cover = ctx->buf<int32_t>("l_cover", (size_t)kLevels * npep1, e);
         if (e) return cuda_fail(ctx, e, "alloc");
         int32_t *partial = ctx->buf<int32_t>("l_partial", hfx_scan_partials_needed(kLevels * npep1), e);
@@ -792,8 +821,8 @@ int32_t search_batched(hfx_ctx *ctx, const hfx_search_params *p, const Batch &b,
             HFX_CUDA(cudaMemsetAsync(stats, 0, 64, ctx->stream), "memset");
         }
         ctx->stage_begin(HFX_STAGE_LISTS);
-        rc = hfx_lists_mark(meta, wb, we, ns, npep1, diff, ctx->stream);
-        if (!rc) rc = hfx_scan_inclusive(diff, kLevels * npep1, cover, partial, ctx->stream);
+        rc = hfx_lists_mark(meta, wb, we, ns, npep1, cover, ctx->stream);
+        if (!rc) rc = hfx_scan_inclusive(cover, kLevels * npep1, cover, partial, ctx->stream);
         if (!rc && long_rows)
             rc = hfx_lists_generate_long(db, cover, npep1, (int32_t)stride, ctx->d_lstart.as<uint32_t>(), total10,
                                          (uint32_t *)lists, llen, work, p->fastdiv,
@@ -967,7 +996,7 @@ int32_t search_batched(hfx_ctx *ctx, const hfx_search_params *p, const Batch &b,
                 ctx->last_open = n_open;
                 if (n_open > 0) {
                     // a plan of these spectra alone over the same lists
-                    rc = hfx_batched_plan(open, ns, wb, we, G, chunk, p->chunk > 0 ? 0 : 1, ws, nullptr, ctx->stream);
+                    rc = hfx_batched_plan(open, ns, wb, we, G, chunk, few_groups, ws, nullptr, ctx->stream);
                     if (rc) return cuda_fail(ctx, (cudaError_t)rc, "plan");
                     uint32_t hs[4];
                     HFX_CUDA(cudaMemcpyAsync(hs, scal, 16, cudaMemcpyDeviceToHost, ctx->stream), "D2H plan");
@@ -1128,7 +1157,7 @@ int32_t search_graph(hfx_ctx *ctx, const hfx_search_params *p, const Batch &b, f
     ctx->cap_groups = (uint32_t)((b.nspec + G - 1) / G + 24);  // <= one partial group per class
     // few groups have more items the wider their windows are, up to kFewItems of
     // each kind beyond what the work-item size alone gives
-    uint32_t items = ctx->last_items + ctx->last_items / 4 + 64 + (p->chunk > 0 ? 0u : 2u * kFewItems);
+    uint32_t items = ctx->last_items + ctx->last_items / 4 + 64 + (p->chunk > 0 || ctx->lean ? 0u : 2u * kFewItems);
     uint32_t tiles = ctx->last_tiles ? ctx->last_tiles + ctx->last_tiles / 4 + 2 : 0;
     uint32_t ditems = ctx->last_ditems ? ctx->last_ditems + ctx->last_ditems / 4 + 64 : 0;
     if (outgrown) {
@@ -1167,6 +1196,18 @@ int32_t search_graph(hfx_ctx *ctx, const hfx_search_params *p, const Batch &b, f
     return restore(HFX_OK);
 }
 
+// Runs a search, and once more in the least room where there was none for it.
+template <typename F>
+int32_t in_room(hfx_ctx *ctx, F run) {
+    const int32_t rc = run();
+    if (rc != HFX_ERR_OOM || ctx->lean) return rc;
+    ctx->drop_search_workspaces();
+    ctx->lean = true;
+    const int32_t again = run();
+    ctx->lean = false;
+    return again;
+}
+
 int32_t search_device(hfx_ctx *ctx, const hfx_search_params *p, const Batch &b, float *out_s, uint64_t *out_k,
                       uint32_t *out_pep, int64_t *out_ncand) {
     int32_t rc = check_params(ctx, p);
@@ -1174,14 +1215,13 @@ int32_t search_device(hfx_ctx *ctx, const hfx_search_params *p, const Batch &b, 
     if (b.nspec <= 0) return HFX_OK;
     HFX_CUDA(cudaSetDevice(ctx->device), "cudaSetDevice");
     HFX_CUDA(ctx->d_err.ensure(16), "alloc err");
-    if (p->use_graph) {
-        if (!p->batch_mode && !(p->search_mods && ctx->num_mod > 0))
-            return fail(ctx, HFX_ERR_UNSUPPORTED, "graph replay needs a batched mode (batch_mode 1 or 2)");
-        return search_graph(ctx, p, b, out_s, out_k, out_pep, out_ncand);
-    }
-    rc = search_enqueue(ctx, p, b, out_s, out_k, out_pep, out_ncand);
-    if (rc) return rc;
-    return search_finish(ctx);
+    if (p->use_graph && !p->batch_mode && !(p->search_mods && ctx->num_mod > 0))
+        return fail(ctx, HFX_ERR_UNSUPPORTED, "graph replay needs a batched mode (batch_mode 1 or 2)");
+    return in_room(ctx, [&] {
+        if (p->use_graph) return search_graph(ctx, p, b, out_s, out_k, out_pep, out_ncand);
+        const int32_t r = search_enqueue(ctx, p, b, out_s, out_k, out_pep, out_ncand);
+        return r ? r : search_finish(ctx);
+    });
 }
 
 }  // namespace
@@ -1592,15 +1632,10 @@ int32_t hfx_search_device(hfx_ctx *ctx, const hfx_search_params *p, const float 
     return search_device(ctx, p, b, out_s, out_k, out_pep, out_ncand);
 }
 
-int32_t hfx_search_evalues(hfx_ctx *ctx, const hfx_search_params *p, const float *mz, const float *it,
-                           const int64_t *off, const float *pcr, const float *z, const float *tol, int32_t nspec,
-                           int32_t bin_width, float cutoff_perc, float *out_s, uint64_t *out_k, uint32_t *out_pep,
-                           int64_t *out_ncand, double *out_ev, double *out_fit) {
-    if (!ctx || !p || nspec < 0 || !out_s || !out_k || !out_ev || !out_fit)
-        return fail(ctx, HFX_ERR_ARG, "bad hfx_search_evalues arguments");
-    if (bin_width < 1 || !(cutoff_perc >= 0.0f && cutoff_perc <= 100.0f))
-        return fail(ctx, HFX_ERR_ARG, "E-value bin width must be >= 1 and the cut-off 0..100 %");
-    if (nspec == 0) return HFX_OK;
+static int32_t search_evalues(hfx_ctx *ctx, const hfx_search_params *p, const float *mz, const float *it,
+                              const int64_t *off, const float *pcr, const float *z, const float *tol, int32_t nspec,
+                              int32_t bin_width, float cutoff_perc, float *out_s, uint64_t *out_k, uint32_t *out_pep,
+                              int64_t *out_ncand, double *out_ev, double *out_fit) {
     const bool mods_on = p->search_mods != 0 && ctx->num_mod > 0;
     const bool plain_on = p->search_plain != 0;
     Batch b{mz, it, pcr, z, tol, off, nspec};
@@ -1681,7 +1716,7 @@ int32_t hfx_search_evalues(hfx_ctx *ctx, const hfx_search_params *p, const float
     ws.group_of = ctx->buf<int32_t>("b_groupof", ns, e);
     ws.slot_of = ctx->buf<int32_t>("b_slotof", ns, e);
     if (e) return cuda_fail(ctx, e, "alloc");
-    rc = hfx_batched_plan(meta, ns, wb, we, G, chunk, p->chunk > 0 ? 0 : 1, ws, nullptr, ctx->stream);
+    rc = hfx_batched_plan(meta, ns, wb, we, G, chunk, p->chunk > 0 || ctx->lean ? 0 : 1, ws, nullptr, ctx->stream);
     if (rc) return cuda_fail(ctx, (cudaError_t)rc, "plan");
     uint32_t hs[4];
     HFX_CUDA(cudaMemcpyAsync(hs, scal, 16, cudaMemcpyDeviceToHost, ctx->stream), "D2H plan");
@@ -1746,6 +1781,21 @@ int32_t hfx_search_evalues(hfx_ctx *ctx, const hfx_search_params *p, const float
     if (!rc) rc = hfx_evalue_apply(out_s, out_k, out_fit, ns, p->top_n, out_ev, ctx->stream);
     if (rc) return cuda_fail(ctx, (cudaError_t)rc, "E-values");
     return search_finish(ctx);
+}
+
+int32_t hfx_search_evalues(hfx_ctx *ctx, const hfx_search_params *p, const float *mz, const float *it,
+                           const int64_t *off, const float *pcr, const float *z, const float *tol, int32_t nspec,
+                           int32_t bin_width, float cutoff_perc, float *out_s, uint64_t *out_k, uint32_t *out_pep,
+                           int64_t *out_ncand, double *out_ev, double *out_fit) {
+    if (!ctx || !p || nspec < 0 || !out_s || !out_k || !out_ev || !out_fit)
+        return fail(ctx, HFX_ERR_ARG, "bad hfx_search_evalues arguments");
+    if (bin_width < 1 || !(cutoff_perc >= 0.0f && cutoff_perc <= 100.0f))
+        return fail(ctx, HFX_ERR_ARG, "E-value bin width must be >= 1 and the cut-off 0..100 %");
+    if (nspec == 0) return HFX_OK;
+    return in_room(ctx, [&] {
+        return search_evalues(ctx, p, mz, it, off, pcr, z, tol, nspec, bin_width, cutoff_perc, out_s, out_k, out_pep,
+                              out_ncand, out_ev, out_fit);
+    });
 }
 
 int32_t hfx_match_ions(hfx_ctx *ctx, const hfx_search_params *p, const float *z, int32_t nspec,

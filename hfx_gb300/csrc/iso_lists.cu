@@ -225,13 +225,15 @@ __device__ __forceinline__ int iso_positions(const DevDB &db, const DevMods &mod
     return list_class(tc, tn);
 }
 
+// Records [first, end).
 __global__ void __launch_bounds__(256) k_iso_positions(DevDB db, DevMods mods, const int32_t *__restrict__ total_p,
-                                                       uint32_t cap_iso, const uint64_t *__restrict__ iso_key,
+                                                       uint32_t first, uint32_t end,
+                                                       const uint64_t *__restrict__ iso_key,
                                                        int32_t pos_words, uint32_t *__restrict__ iso_pos,
                                                        WorkLists wl, uint16_t *__restrict__ iso_len,
                                                        uint32_t *__restrict__ err) {
-    const uint32_t total = min((uint32_t)*total_p, cap_iso);
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t total = min((uint32_t)*total_p, end);
+    const uint32_t t = first + blockIdx.x * blockDim.x + threadIdx.x;
     int cls = -1;
     if (t < total) {
         cls = iso_positions(db, mods, iso_key[t], t, pos_words, iso_pos, err);
@@ -626,16 +628,14 @@ int hfx_iso_expand(const DevDB &db, const DevMods &m, const int32_t *cover, cons
 int hfx_iso_generate(const DevDB &db, const DevMods &m, const int32_t *cover, int32_t nbins, const uint32_t *lstart,
                      const int32_t *total_p, uint32_t cap_iso, const uint64_t *iso_key, const uint64_t *iso_off,
                      uint16_t *lists, uint64_t list_total, uint16_t *iso_len, int32_t pos_words,
-                     uint32_t *iso_pos, uint32_t *work, int fastdiv, unsigned long long *stats, uint32_t *err,
-                     cudaStream_t st) {
+                     uint32_t *iso_pos, uint32_t *work, uint64_t work_cap, int fastdiv, unsigned long long *stats,
+                     uint32_t *err, cudaStream_t st) {
     if (cap_iso == 0) return 0;
+    if (work_cap == 0) return (int)cudaErrorInvalidValue;
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const WorkLists wl{work, cap_iso};
-    cudaMemsetAsync(work, 0, 16, st);
-    k_iso_positions<<<(unsigned)(((uint64_t)cap_iso + 255) / 256), 256, 0, st>>>(
-        db, m, total_p, cap_iso, iso_key, pos_words, iso_pos, wl, iso_len, err);
+    const WorkLists wl{work, work_cap};
     auto run = [&](auto f, int cls) {
         const size_t smem = (size_t)(256 / class_lanes(cls)) * rank_bytes(nbins, cls);
         // (the longest rows': see hfx_lists_generate)
@@ -647,10 +647,16 @@ int hfx_iso_generate(const DevDB &db, const DevMods &m, const int32_t *cover, in
             db, m, cover, (int64_t)db.num_pep + 1, nbins, lstart, iso_key, iso_off, lists, list_total, iso_len,
             pos_words, iso_pos, wl, stats, err);
     };
-    run(fastdiv ? k_gen_iso_lists<true, 3> : k_gen_iso_lists<false, 3>, 3);
-    run(fastdiv ? k_gen_iso_lists<true, 1> : k_gen_iso_lists<false, 1>, 1);
-    run(fastdiv ? k_gen_iso_lists<true, 2> : k_gen_iso_lists<false, 2>, 2);
-    run(fastdiv ? k_gen_iso_lists<true, 0> : k_gen_iso_lists<false, 0>, 0);
+    for (uint64_t first = 0; first < cap_iso; first += work_cap) {
+        const uint64_t some = std::min<uint64_t>(work_cap, cap_iso - first);
+        cudaMemsetAsync(work, 0, 16, st);
+        k_iso_positions<<<(unsigned)((some + 255) / 256), 256, 0, st>>>(
+            db, m, total_p, (uint32_t)first, (uint32_t)(first + some), iso_key, pos_words, iso_pos, wl, iso_len, err);
+        run(fastdiv ? k_gen_iso_lists<true, 3> : k_gen_iso_lists<false, 3>, 3);
+        run(fastdiv ? k_gen_iso_lists<true, 1> : k_gen_iso_lists<false, 1>, 1);
+        run(fastdiv ? k_gen_iso_lists<true, 2> : k_gen_iso_lists<false, 2>, 2);
+        run(fastdiv ? k_gen_iso_lists<true, 0> : k_gen_iso_lists<false, 0>, 0);
+    }
     return (int)cudaGetLastError();
 }
 

@@ -24,13 +24,14 @@ int hfx_iso_expand(const hfx::DevDB &db, const hfx::DevMods &m, const int32_t *c
 // needed level; iso_len [isoform][kLevels].  total_p: the device total.
 // First the residues each isoform modifies (iso_pos, pos_words words per
 // record, at least the longest peptide's residues / 32).
-// work: hfx_lists_work_words(cap_iso) words of scratch.
+// work: hfx_lists_work_words(work_cap) words of scratch; the
+// records are taken work_cap at a time.
 // stats (nullable, 8 counters): [0] lists, [1] entries, [5] isoform records,
 // [6] residues read.
 int hfx_iso_generate(const hfx::DevDB &db, const hfx::DevMods &m, const int32_t *cover, int32_t nbins,
                      const uint32_t *lstart, const int32_t *total_p, uint32_t cap_iso, const uint64_t *iso_key,
                      const uint64_t *iso_off, uint16_t *lists, uint64_t list_total, uint16_t *iso_len,
-                     int32_t pos_words, uint32_t *iso_pos, uint32_t *work, int fastdiv,
+                     int32_t pos_words, uint32_t *iso_pos, uint32_t *work, uint64_t work_cap, int fastdiv,
                      unsigned long long *stats, uint32_t *err, cudaStream_t st);
 // The scorer over the isoform lists and the group tiles; work items and
 // partial outputs as hfx_mods_score's (without a score sink).  stats

@@ -735,6 +735,7 @@ int hfx_lists_mark(const SpecMeta *meta, const uint32_t *wb, const uint32_t *we,
 }
 
 size_t hfx_lists_work_words(uint64_t n) { return work_words(n); }
+uint64_t hfx_lists_work_cap(uint64_t words) { return words > work_words(0) ? (words - work_words(0)) / kWorkLists : 0; }
 
 int hfx_lists_generate(const DevDB &db, const int32_t *cover, int64_t npep1, int32_t nbins, const uint32_t *lstart,
                        uint64_t total10, uint16_t *lists, uint16_t *list_len, uint32_t *work, int fastdiv,

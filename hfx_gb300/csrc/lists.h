@@ -21,6 +21,7 @@ int hfx_lists_generate(const hfx::DevDB &db, const int32_t *cover, int64_t npep1
                        const uint32_t *lstart, uint64_t total10, uint16_t *lists, uint16_t *list_len,
                        uint32_t *work, int fastdiv, unsigned long long *stats, cudaStream_t st);
 size_t hfx_lists_work_words(uint64_t n);
+uint64_t hfx_lists_work_cap(uint64_t words);  // entries that so many words hold
 // Scorer over the lists; long_rows: 32-bit entries and group tiles read
 // from global memory (rows too long for shared memory), else 16-bit entries
 // and tiles staged in shared memory.
