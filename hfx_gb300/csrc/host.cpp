@@ -609,8 +609,8 @@ int32_t search_isoform_lists(hfx_ctx *ctx, const hfx_search_params *p, const Spe
                               len, pos_words, pos, work, work_cap, p->fastdiv, stats, ctx->d_err.as<uint32_t>(),
                               ctx->stream);
     if (rc) return cuda_fail(ctx, (cudaError_t)rc, "isoform lists");
-    // windows, planning, 9 isoform-list kernels and 5 for each run of records
-    ctx->stage_end(HFX_STAGE_MOD_LISTS, 14 + 5 * (int64_t)((cap_iso + work_cap - 1) / std::max<uint64_t>(work_cap, 1)),
+    // windows, 4 of planning, 11 of hfx_iso_plan, k_iso_expand, and 5 for each run of records
+    ctx->stage_end(HFX_STAGE_MOD_LISTS, 17 + 5 * (int64_t)((cap_iso + work_cap - 1) / std::max<uint64_t>(work_cap, 1)),
                    (int64_t)cap_iso);
     ctx->stage_begin(HFX_STAGE_MODS);
     rc = hfx_iso_score(lists, cap_entries, ctx->d_lstart.as<uint32_t>(), key, off, len, count, incl,
@@ -721,7 +721,7 @@ int32_t search_batched(hfx_ctx *ctx, const hfx_search_params *p, const Batch &b,
     rc = hfx_batched_plan(meta, ns, wb, we, G, chunk, few_groups, ws, dense_on ? &dw : nullptr, ctx->stream);
     if (rc) return cuda_fail(ctx, (cudaError_t)rc, "plan");
     // k_windows + the planning kernels
-    ctx->stage_end(HFX_STAGE_WINDOWS, (dense_on ? 8 : 6) - (ns <= kSortFew ? 2 : 0), ns);
+    ctx->stage_end(HFX_STAGE_WINDOWS, (dense_on ? 9 : 6) - (ns <= kSortFew ? 2 : 0), ns);
     uint32_t ngroups = 0, total_items = 0, ntiles = 0, ditems = 0;
     if (ctx->gmode >= 1) {
         // capacities of the graph; a batch that needs more is reported (k_clamp_items)
@@ -833,7 +833,8 @@ int32_t search_batched(hfx_ctx *ctx, const hfx_search_params *p, const Batch &b,
                                     ctx->d_lstart.as<uint32_t>(), total10, (uint16_t *)lists, llen, work,
                                     p->fastdiv, stats, ctx->stream);
         if (rc) return cuda_fail(ctx, (cudaError_t)rc, "ion lists");
-        ctx->stage_end(HFX_STAGE_LISTS, 8, 0);  // mark, 3 scans, k_list_work, 3 classes of k_gen_lists
+        // mark, 3 scans, k_list_work and the classes: 4 of k_gen_lists, 3 of k_gen_lists_long
+        ctx->stage_end(HFX_STAGE_LISTS, long_rows ? 8 : 9, 0);
         ctx->stage_begin(HFX_STAGE_SCORE);
         float *sink = nullptr;
         const uint64_t *sink_off = nullptr;
@@ -861,8 +862,8 @@ int32_t search_batched(hfx_ctx *ctx, const hfx_search_params *p, const Batch &b,
         if (rc) return cuda_fail(ctx, (cudaError_t)rc, "k_score_lists");
         if (dtiles) {
             rc = hfx_dense_score((const uint16_t *)lists, total10 * 10, ctx->d_lstart.as<uint32_t>(), total10, llen,
-                                 (uint32_t)ctx->num_pep, dtiles, ntiles, stride, pieces, wb, we, ns, ws, dw, K,
-                                 stats, ctx->d_err.as<uint32_t>(), ctx->stream);
+                                 (uint32_t)ctx->num_pep, dtiles, ntiles, stride, pieces, wb, we, ws, dw, K, stats,
+                                 ctx->d_err.as<uint32_t>(), ctx->stream);
             if (rc) return cuda_fail(ctx, (cudaError_t)rc, "k_dense_score");
         }
         ctx->stage_end(HFX_STAGE_SCORE, dtiles ? 2 : 1, 0);
