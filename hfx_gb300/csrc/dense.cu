@@ -78,7 +78,9 @@ __host__ __device__ __forceinline__ uint32_t swizzled(uint32_t r, uint32_t k) {
 // 0.64 ns whatever the block's windows (18 M rows in 10.5 ms), a pair of the list
 // scorer 0.038 ns.  With the line at 16 the +-3 Da blocks of 10,000 spectra that
 // passed it made their scoring slower (2.78 -> 3.15 ms); at 32 none of them does,
-// and open windows have 36 to 115 (kDenseMinPairs).
+// and open windows have 36 to 115 (kDenseMinPairs).  A union of fewer than eight
+// passes is left to the list scorer too: its pairs with 128 spectra take that
+// 20 us, as long as one pass of an SM.
 constexpr uint32_t kDenseMinWidth = 4096;
 
 __global__ void k_dense_clear(DenseWs dw, int32_t nspec) {
@@ -839,10 +841,8 @@ int hfx_dense_pack(const float *rows, int64_t stride, const BatchedWs &ws, const
 
 int hfx_dense_score(const uint16_t *lists, uint64_t list_total, const uint32_t *lstart, uint64_t total10,
                     const uint16_t *list_len, uint32_t num_pep, const uint8_t *tiles, uint32_t cap_tiles,
-                    int64_t stride, int pieces, const uint32_t *wb, const uint32_t *we, int32_t nspec,
-                    const BatchedWs &ws, const DenseWs &dw, int32_t K, unsigned long long *stats, uint32_t *err,
-                    cudaStream_t st) {
-    (void)nspec;
+                    int64_t stride, int pieces, const uint32_t *wb, const uint32_t *we, const BatchedWs &ws,
+                    const DenseWs &dw, int32_t K, unsigned long long *stats, uint32_t *err, cudaStream_t st) {
     if (cap_tiles == 0) return 0;
     if (K > 32) return (int)cudaErrorInvalidValue;
     int dev = 0, sms = 0;

@@ -57,9 +57,8 @@ int hfx_dense_pack(const float *rows, int64_t stride, const hfx::BatchedWs &ws, 
                    uint32_t cap_tiles, int pieces, uint8_t *tiles, uint32_t *err, cudaStream_t st);
 int hfx_dense_score(const uint16_t *lists, uint64_t list_total, const uint32_t *lstart, uint64_t total10,
                     const uint16_t *list_len, uint32_t num_pep, const uint8_t *tiles, uint32_t cap_tiles,
-                    int64_t stride, int pieces, const uint32_t *wb, const uint32_t *we, int32_t nspec,
-                    const hfx::BatchedWs &ws, const hfx::DenseWs &dw, int32_t K, unsigned long long *stats, uint32_t *err,
-                    cudaStream_t st);
+                    int64_t stride, int pieces, const uint32_t *wb, const uint32_t *we, const hfx::BatchedWs &ws,
+                    const hfx::DenseWs &dw, int32_t K, unsigned long long *stats, uint32_t *err, cudaStream_t st);
 // FP32 searches, after the rescoring: of each spectrum of a dense block, whether
 // its out_s[topn] certainly hold its best candidates (dense.cu).  open_meta: meta
 // with a status other than 0 for every spectrum that needs nothing more;

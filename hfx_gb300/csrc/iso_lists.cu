@@ -19,10 +19,10 @@
 //      rank; Search.hs:119-123) and its slot;
 //   4. one thread per isoform: unrank the modified residues
 //      (gen_mod_pep.cu:127-227, combinatorics.h:90-134) into a bit per
-//      residue; then one warp per isoform: build the bit planes of charges
-//      1..zmax with the modified masses (residual + delta, residue mass +
-//      acid delta) and write the distinct-bin list of every needed level
-//      (the list format of lists.cu);
+//      residue; then half a warp or a warp per isoform, by the length of its
+//      ladder: the distinct-bin list of every needed level from the modified
+//      masses (residual + delta, residue mass + acid delta), each entry at its
+//      rank among the level's bins (lists_device.cuh; the format of lists.cu);
 //   5. the scorer: work items (spectrum group, combination, chunk of
 //      positions) as in the fused path; an item's isoforms are a contiguous
 //      index range; each is streamed against the group's tile.

@@ -62,11 +62,6 @@ __device__ __forceinline__ RankBufs rank_bufs(const uint8_t *base, int32_t nbins
     return rb;
 }
 
-__device__ __forceinline__ uint32_t lds_u16(uint32_t a) {
-    uint16_t v;
-    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(a) : "memory");
-    return v;
-}
 __device__ __forceinline__ uint32_t lds_u32(uint32_t a) {
     uint32_t v;
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
@@ -172,8 +167,9 @@ struct ItemBits {
 // remainder a - q d is exact in one FMA, and q + remainder y rounds to the
 // quotient (Markstein, IBM J. Res. Dev. 34, 1990).  Equal to the IEEE division
 // for d = 1.0005079, 0.02 and 3 and every float in [2^-12, 2^22], which is where
-// the ions lie (tests/test_lists_math.py; an infinite a would give a NaN, so
-// masses from 2^22 on take the other path).  Three instructions and no branch;
+// the ions lie (all of them compared once with the division;
+// tests/test_lists_math.py compares some of them in exact arithmetic.  An
+// infinite a would give a NaN, so masses from 2^22 on take the other path).  Three instructions and no branch;
 // the division's own slow path is a call, which costs a kernel that keeps a
 // candidate in registers 16 of them and spills.
 __device__ __forceinline__ float quotient(float a, float d, float y) {

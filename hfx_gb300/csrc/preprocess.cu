@@ -83,7 +83,6 @@ __global__ void k_layout(const float *__restrict__ mz, const int64_t *__restrict
     if (m.status == 0) atomicMax(max_len, (uint32_t)m.len);
 }
 
-// One CTA per spectrum; the whole row sits in shared memory.
 // Block-wide exclusive scan of one value per thread (blockDim.x <= 1024).
 __device__ __forceinline__ int32_t block_excl_scan(int32_t v, int32_t *warp_tot, int32_t &total) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
