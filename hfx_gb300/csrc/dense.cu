@@ -605,6 +605,7 @@ k_dense_score(const uint16_t *__restrict__ lists, uint64_t list_total, const uin
                     }
                     if (fresh) floor_key = (unsigned long long)score_order(low) << 32;
                 }
+                float cut = cut_from(pb);
 #pragma unroll 1
                 for (uint32_t j0 = 0; j0 < kDenseRows; j0 += 32) {
                     float v[32];
@@ -614,7 +615,6 @@ k_dense_score(const uint16_t *__restrict__ lists, uint64_t list_total, const uin
                     for (int j = 1; j < 30; j += 2) top = max_nan(top, v[j], v[j + 1]);
                     // this spectrum's columns of these 32
                     const uint32_t from = c0 > j0 ? min(c0 - j0, 32u) : 0u, to = c1 > j0 ? min(c1 - j0, 32u) : 0u;
-                    const float cut = cut_from(pb + j0);
                     if (!__any_sync(kFullMask, to > from && !(top < cut))) continue;
                     uint32_t hit = 0;
 #pragma unroll
@@ -628,9 +628,9 @@ k_dense_score(const uint16_t *__restrict__ lists, uint64_t list_total, const uin
                         if (((hit >> j) & 1u) && x > floor_key) q[m * kDenseQueue + qn++] = x;
                         uint32_t full = __ballot_sync(kFullMask, qn == (uint32_t)kDenseQueue);
                         __syncwarp();
-                        while (full) {
-                            merge(__ffs(full) - 1);
-                            full &= full - 1u;
+                        if (full) {
+                            for (; full; full &= full - 1u) merge(__ffs(full) - 1);
+                            cut = cut_from(pb);
                         }
                     }
                 }
