@@ -679,13 +679,16 @@ int32_t search_batched(hfx_ctx *ctx, const hfx_search_params *p, const Batch &b,
     uint32_t *scal = ctx->buf<uint32_t>("b_scal", 8, e);
     if (e) return cuda_fail(ctx, e, "alloc");
     // wide windows on the tensor cores: unmodified candidates, lists, up to 32
-    // kept, and without a score sink; an FP32 search keeps 32 then and rescores
-    // them, so it has to ask for few enough of them, and the spectra whose results
-    // are not certain then (hfx_dense_prove) are list-scored below.  A block's pairs
+    // kept, and without a score sink.  Their scores choose what is rescored, so at
+    // least as many candidates more have to be kept as results are asked for (an
+    // FP32 search keeps 32 then); without them another rounding would be another
+    // result.  FP32 spectra whose results are not certain even so (hfx_dense_prove)
+    // are list-scored below.  A block's pairs
     // are at most its spectra times their union, so fewer spectra than the rule's
     // share have no block and need no plan of them (15 us of a one-spectrum search)
     const bool dense_on = lists_only && !long_rows && K <= 32 && p->search_plain != 0 && ns >= kDenseMinPairs &&
-                          !ctx->lean && (elem_kind != 0 || (p->top_n <= 16 && !ctx->ev_single && ctx->dense_fp32));
+                          !ctx->lean && p->top_n <= (elem_kind != 0 ? K : kMaxTopK) / 2 &&
+                          (elem_kind != 0 || (!ctx->ev_single && ctx->dense_fp32));
     DenseWs dw{};
     if (dense_on) {
         dw.cap_blocks = dense_blocks(ns);

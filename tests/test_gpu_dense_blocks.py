@@ -40,3 +40,19 @@ def test_blocks(engine, oracle, precision, charges, launches):
     assert np.array_equal(res.ncand, nc)
     assert np.array_equal(res.key, key)
     assert np.array_equal(res.score.view(np.uint32), sc.view(np.uint32))
+
+
+@pytest.mark.parametrize("precision,top_n,rescore_k,launches", [
+    (1, 16, 32, 2), (1, 17, 32, 1), (1, 16, 10, 1), (2, 10, 20, 2), (2, 10, 19, 1), (0, 16, 0, 2), (0, 17, 0, 1)])
+def test_candidates_to_spare(engine, precision, top_n, rescore_k, launches):
+    """The tensor cores choose candidates only where twice the results are kept."""
+    import hfx_gb300
+    eng, prot = engine
+    sp = synth.spectra(prot, 64, seed=64, charge_p={2: 1.0}, npeaks=(50, 200))
+    sp.tol[:] = 1e5
+    eng.set_profiling(True)
+    eng.stage_stats()
+    eng.search(sp, hfx_gb300.default_params(top_n=top_n, batch_mode=1, precision=precision, rescore_k=rescore_k))
+    seen = eng.stage_stats()["score"][1]
+    eng.set_profiling(False)
+    assert seen == launches
