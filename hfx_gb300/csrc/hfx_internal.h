@@ -26,9 +26,12 @@ struct LayoutParams {
 struct SpecMeta {
     int32_t npk, len, status;
     float cutoff, mass, eps, lo, hi;
-    int32_t charges_plain, charges_mod;
-    int32_t nonfinite;  // a kept peak's intensity is infinite (its row holds NaN)
+    int32_t charges_plain;
+    int16_t charges_mod;
+    int16_t nonfinite;  // a kept peak's intensity is infinite (its row holds NaN)
 };
+// a search's workspace per spectrum, which callers' limits count on
+static_assert(sizeof(SpecMeta) == 40, "a spectrum's workspace has grown");
 
 // Search database on the device, in residual-mass order.
 struct DevDB {

@@ -75,7 +75,7 @@ __global__ void k_layout(const float *__restrict__ mz, const int64_t *__restrict
     const float rr = rintf(mc);
     int32_t ch = (rr >= 1.0f) ? (rr > 1000.0f ? 1000 : (int32_t)rr) : 0;
     m.charges_plain = (ch >= 1 && ch <= 4) ? ch : 0;
-    m.charges_mod = (ch >= 1 && ch <= 10) ? min(ch, 4) : 0;  // mion_series.cu:303-306, 425-438
+    m.charges_mod = (int16_t)((ch >= 1 && ch <= 10) ? min(ch, 4) : 0);  // mion_series.cu:303-306, 425-438
     m.nonfinite = 0;
     meta[s] = m;
     if (lens) lens[s] = m.status == 0 ? m.len : 0;
