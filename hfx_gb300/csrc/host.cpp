@@ -152,6 +152,7 @@ struct hfx_ctx {
     uint32_t last_tiles = 0, cap_tiles = 0, last_ditems = 0, cap_ditems = 0;  // dense blocks: operand tiles, items
     uint32_t last_open = 0;     // FP32 spectra whose dense results were not certain
     bool dense_fp32 = true;     // off while a graph is made of a batch that has such spectra
+    bool graph_lists = false;   // the captured graph was
     bool graph_valid = false;
     cudaGraphExec_t graph_exec = nullptr;
     cudaStream_t graph_stream = nullptr;  // captures and replays run here (never the legacy stream)
@@ -1145,6 +1146,8 @@ int32_t search_graph(hfx_ctx *ctx, const hfx_search_params *p, const Batch &b, f
     };
     ctx->gmode = 0;
     ctx->last_open = 0;
+    // (and is made so again, or batches with and without them would take turns)
+    if (outgrown && ctx->graph_lists) ctx->dense_fp32 = false;
     int32_t rc = search_enqueue(ctx, p, b, out_s, out_k, out_pep, out_ncand);
     if (!rc) rc = search_finish(ctx);
     if (!rc && ctx->last_open > 0) {
@@ -1197,6 +1200,7 @@ int32_t search_graph(hfx_ctx *ctx, const hfx_search_params *p, const Batch &b, f
     }
     ctx->graph_valid = true;
     ctx->graph_key = key;
+    ctx->graph_lists = !ctx->dense_fp32;
     return restore(HFX_OK);
 }
 
