@@ -67,17 +67,17 @@ KERNEL_SRC = {
 # per-kernel basis below) to the small case's.
 TRAFFIC = {
     ("k_gen_lists", "full", 1, 10000): {
-        "src": "2c86f8c5f15c", "bytes": 1969009253, "inst": 1909988937,
+        "src": "a406d6e61dc2", "bytes": 1968937107, "inst": 1909988643,
         "profile": "profiles/k_gen_lists_2k_bf16.md (2,000-spectrum capture x 1.729 moved-bytes ratio)"},
     ("k_score_lists", "full", 1, 10000): {
-        "src": "2c86f8c5f15c", "bytes": 3320183081, "inst": 2170058895,
-        "profile": "profiles/k_score_lists_2k_bf16.md (2,000-spectrum capture x 2.482 moved-bytes ratio)"},
+        "src": "a406d6e61dc2", "bytes": 3318507544, "inst": 2167953456,
+        "profile": "profiles/k_score_lists_2k_bf16.md (2,000-spectrum capture x 2.480 moved-bytes ratio)"},
     ("k_gen_iso_lists", "mods", 1, 10000): {
-        "src": "606c66706d60", "bytes": 50460321735, "inst": 56449742430,
+        "src": "634b54d03f7a", "bytes": 50467129798, "inst": 56450310718,
         "profile": "profiles/iso_lists_mods_bf16.md (500-spectrum capture x 6.986 moved-bytes ratio)"},
     ("k_score_iso_lists", "mods", 1, 10000): {
-        "src": "606c66706d60", "bytes": 74375970086, "inst": 38759597972,
-        "profile": "profiles/iso_lists_mods_bf16.md (500-spectrum capture x 10.258 moved-bytes ratio)"},
+        "src": "634b54d03f7a", "bytes": 74381598276, "inst": 38761859384,
+        "profile": "profiles/iso_lists_mods_bf16.md (500-spectrum capture x 10.259 moved-bytes ratio)"},
 }
 
 

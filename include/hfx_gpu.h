@@ -90,7 +90,9 @@ int32_t hfx_set_profiling(hfx_ctx *ctx, int32_t on);
  * sizes its dense matrices to the free memory, Search.hs:427-433): a call
  * whose workspaces would grow the context beyond `bytes` allocates nothing
  * more and returns HFX_ERR_OOM, and the context stays usable (raise the cap
- * and call again).  0 = no cap.  in_use (nullable) receives the bytes held
+ * and call again).  A search (E-values included) first frees what earlier
+ * searches left and runs once more without the workspaces that help speed
+ * alone; its results are the same.  0 = no cap.  in_use (nullable) receives the bytes held
  * now.  The database and the per-call host staging are not counted. */
 int32_t hfx_set_workspace_limit(hfx_ctx *ctx, uint64_t bytes, uint64_t *in_use);
 int32_t hfx_stage_stats(hfx_ctx *ctx, double *ms, int64_t *launches, int64_t *units, int32_t reset);
