@@ -40,7 +40,7 @@
 // offer what reaches the spectrum's threshold to its list of the best K.
 //
 // Measured (20,000 proteins, 80 % +-10 ppm and 20 % +-500 Da windows, all
-// scoring): 20,000 spectra in BF16 70.1 -> 13.1 ms, 3,001 in FP32 24.4 -> 14.1 ms.
+// scoring): 20,000 spectra in BF16 70.1 -> 13.5 ms, 3,001 in FP32 24.4 -> 13.5 ms.
 // A chunk takes about 5,700 cycles, 2,050 of them MMAs (6,100 of FP32's six
 // pieces): spreading the lists bounds the rest, its byte stores and list loads
 // (3,200 shared-memory cycles), then the epilogue (a quarter).
